@@ -137,6 +137,14 @@ __global__ void k_pack(MolDev m, const int* __restrict__ order, int n, float4* _
     rorig[k] = i;
 }
 
+__global__ void k_interleave(const float4* __restrict__ pos, const float4* __restrict__ par, int n,
+                             float4* __restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k > n) return;
+    out[2 * (size_t)k] = k < n ? pos[k] : make_float4(3e30f, 3e30f, 3e30f, 0.f);
+    out[2 * (size_t)k + 1] = k < n ? par[k] : make_float4(0.f, 0.f, 0.f, 1.f);
+}
+
 template <class T>
 cudaError_t up(DBuf& b, const std::vector<T>& v, cudaStream_t s) {
     cudaError_t e = b.reserve(std::max<size_t>(v.size(), 1) * sizeof(T));
@@ -145,6 +153,11 @@ cudaError_t up(DBuf& b, const std::vector<T>& v, cudaStream_t s) {
 }
 
 }  // namespace
+
+cudaError_t interleave_atoms(const float4* pos, const float4* par, int n, float4* out, cudaStream_t s) {
+    k_interleave<<<(unsigned)(n / 256 + 1), 256, 0, s>>>(pos, par, n, out);
+    return cudaGetLastError();
+}
 
 // The receptor's cell-sorted device arrays and cell_start (ncell + 1), built
 // on the GPU for grid origin o, cells nc (x counts sub-cells) and inverse

@@ -7,6 +7,8 @@
 //   [cell_start[row+cx0], cell_start[row+cx1+1]);
 //     rpos  float4 (x, y, z, q)              rpos64 double4 (same, f64)
 //     rpar  float4 (sqrt eps, r, heavy, excl) rpar64 double4 (sqrt eps, r, eps, heavy)
+//     rpk   both float4 of an atom side by side (32 bytes, one load), and
+//           one more atom far from everything
 //     rsolv float2 (des, asa)                rsolv64 double2
 //   ligand atoms ordered by recursive coordinate bisection of the reference
 //   frame into groups of `group` atoms (groups and tiles of consecutive
@@ -32,6 +34,7 @@ struct ComplexDev {
     // receptor (sorted by fine cell)
     const float4* rpos;
     const float4* rpar;
+    const float4* rpk;       // rpos and rpar interleaved: 2 float4 an atom
     const float2* rsolv;
     const double4* rpos64;
     const double4* rpar64;
@@ -55,6 +58,7 @@ struct ComplexDev {
     int rlbx, rlby, rlbz;
     float rlbox, rlboy, rlboz, rlb_inv, rlb_m;
     const float4* lgrp;      // per group of `group` atoms: ligand-frame centre, radius
+    const float4* lquad;     // per 4 consecutive atoms: ligand-frame centre, radius
     int group;               // ligand atoms per candidate-search group
     int ntiles;              // ceil(nl / tile)
     // far field: fnx x fny x fnz points in bricks of 4 x 4 x 4 (fbx x fby x
@@ -125,6 +129,7 @@ struct LaunchParams {
     // (SPILL_SLOT_BYTES each), all slots empty between poses; null: none
     unsigned char* spill;
     int spill_cap;
+    float one;                   // 1.f (warp kernels: a factor the compiler does not know)
     // plain warp kernel: stage candidates in shared memory by bulk copies
     int stage;
     // [N] far-field term of each pose from k_far_poses (fast cpydock

@@ -7,25 +7,30 @@ namespace lkg {
 // outputs are requested (cuda_full_score)
 template <int G>
 static size_t warp_smem(bool stage = false) {
-    return (size_t)(WK_THREADS / 32) * (sizeof(WSlots<G>) + sizeof(WQueue) + (stage ? sizeof(WStage) : 0));
+    return (size_t)(WK_THREADS / 32) * (sizeof(WSlots<G>) + (stage ? sizeof(WStage) : 0));
 }
 
 // IFACE: the variant that also collects the interface bits (launches with
 // restraint or membrane complexes); STAGE: candidates staged in shared
 // memory by bulk copies (contexts that ask for it)
-template <int G, bool IFACE, bool STAGE>
+template <int G, bool IFACE, bool NP, bool STAGE>
 static cudaError_t launch_warp_gi(const LaunchParams& p, int blocks, cudaStream_t s) {
     const size_t sm = warp_smem<G>(STAGE);
-    cudaError_t e = cudaFuncSetAttribute(k_score_warp<G, IFACE, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_score_warp<G, IFACE, NP, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)sm);
     if (e != cudaSuccess) return e;
-    k_score_warp<G, IFACE, STAGE><<<blocks, WK_THREADS, sm, s>>>(p);
+    k_score_warp<G, IFACE, NP, STAGE><<<blocks, WK_THREADS, sm, s>>>(p);
     return cudaGetLastError();
 }
+// near pairs are counted only where the caller takes the parts
 template <int G>
 static cudaError_t launch_warp_g(const LaunchParams& p, int blocks, cudaStream_t s) {
-    if (p.iface) return launch_warp_gi<G, true, false>(p, blocks, s);
-    return p.stage ? launch_warp_gi<G, false, true>(p, blocks, s) : launch_warp_gi<G, false, false>(p, blocks, s);
+    if (p.iface)
+        return p.parts ? launch_warp_gi<G, true, true, false>(p, blocks, s)
+                       : launch_warp_gi<G, true, false, false>(p, blocks, s);
+    if (p.stage) return launch_warp_gi<G, false, true, true>(p, blocks, s);
+    return p.parts ? launch_warp_gi<G, false, true, false>(p, blocks, s)
+                   : launch_warp_gi<G, false, false, false>(p, blocks, s);
 }
 
 cudaError_t launch_score_fast(const LaunchParams& p, int threads, int blocks, cudaStream_t s) {
@@ -46,8 +51,8 @@ template <int G>
 static int occ_warp_g() {
     int m = 0;
     const size_t sm = warp_smem<G>();
-    cudaFuncSetAttribute(k_score_warp<G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_score_warp<G, false>, WK_THREADS, sm);
+    cudaFuncSetAttribute(k_score_warp<G, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_score_warp<G, false, false>, WK_THREADS, sm);
     return m;
 }
 
@@ -55,19 +60,22 @@ size_t desolv_smem_bytes(int hcap, bool /*exact*/) { return (size_t)hcap * 12; }
 
 // cpydock: the warp kernel for group sizes up to 16 (its per-warp slots and
 // the block's minimum hash fit in shared memory), the per-atom kernel above
-template <int G, bool IFACE>
+template <int G, bool IFACE, bool NP>
 static cudaError_t launch_warp_desolv_gi(const LaunchParams& p, int blocks, int hcap, cudaStream_t s) {
     const size_t sm = wd_smem<G>(hcap);
-    cudaError_t e = cudaFuncSetAttribute(k_score_warp_desolv<G, IFACE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sm);
+    cudaError_t e = cudaFuncSetAttribute(k_score_warp_desolv<G, IFACE, NP>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_score_warp_desolv<G, IFACE><<<blocks, WD_THREADS, sm, s>>>(p);
+    k_score_warp_desolv<G, IFACE, NP><<<blocks, WD_THREADS, sm, s>>>(p);
     return cudaGetLastError();
 }
 template <int G>
 static cudaError_t launch_warp_desolv_g(const LaunchParams& p, int blocks, int hcap, cudaStream_t s) {
-    return p.iface ? launch_warp_desolv_gi<G, true>(p, blocks, hcap, s)
-                   : launch_warp_desolv_gi<G, false>(p, blocks, hcap, s);
+    if (p.iface)
+        return p.parts ? launch_warp_desolv_gi<G, true, true>(p, blocks, hcap, s)
+                       : launch_warp_desolv_gi<G, true, false>(p, blocks, hcap, s);
+    return p.parts ? launch_warp_desolv_gi<G, false, true>(p, blocks, hcap, s)
+                   : launch_warp_desolv_gi<G, false, false>(p, blocks, hcap, s);
 }
 
 cudaError_t launch_far_poses(const LaunchParams& p, int blocks, cudaStream_t s) {
@@ -93,8 +101,8 @@ template <int G>
 static int occ_warp_desolv_g(int hcap) {
     int n = 0;
     const size_t sm = wd_smem<G>(hcap);
-    cudaFuncSetAttribute(k_score_warp_desolv<G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_score_warp_desolv<G, false>, WD_THREADS, sm);
+    cudaFuncSetAttribute(k_score_warp_desolv<G, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_score_warp_desolv<G, false, false>, WD_THREADS, sm);
     return n;
 }
 

@@ -179,6 +179,17 @@ std::vector<float> receptor_distance_bound(const double* c, int n, int dims[3], 
 
 namespace {
 
+// rpk from rpos and rpar (both float4 of an atom side by side), then an atom
+// out of reach of everything that adds nothing (it pads the candidate lists)
+int interleave_receptor(lkg_ctx* ctx, ComplexRec& cr, int n) {
+    LKG_CK(cr.rpk.reserve(((size_t)n + 1) * 2 * sizeof(float4)), "receptor arrays");
+    LKG_CK(interleave_atoms(cr.rpos.as<float4>(), cr.rpar.as<float4>(), n, cr.rpk.as<float4>(), ctx->stream),
+           "receptor arrays");
+    ctx->launches++;
+    LKG_CK(cudaStreamSynchronize(ctx->stream), "receptor arrays");
+    return 0;
+}
+
 // receptor: sort by fine cell (x fastest), pack device arrays; the sort and
 // packing run on the GPU (lkg_cells.cu) unless the context asks for the
 // host build
@@ -251,7 +262,9 @@ int build_receptor(lkg_ctx* ctx, const MolIn& R, ComplexRec& cr) {
         LKG_CK(upload(cr.cell_start, cs, s), "upload receptor");
         LKG_CK(cudaStreamSynchronize(s), "upload receptor");
     }
+    if (const int st = interleave_receptor(ctx, cr, n)) return st;
     d.nr = n;
+    d.rpk = cr.rpk.as<float4>();
     d.rpos = cr.rpos.as<float4>(); d.rpar = cr.rpar.as<float4>(); d.rsolv = cr.rsolv.as<float2>();
     d.rpos64 = cr.rpos64.as<double4>(); d.rpar64 = cr.rpar64.as<double4>(); d.rsolv64 = cr.rsolv64.as<double2>();
     d.rorig = cr.rorig.as<int>(); d.cell_start = cr.cell_start.as<int>();
@@ -317,6 +330,8 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
     bisect_groups(L.c.data(), order.data(), n, ctx->group);
+    for (int k = 0; k < n; k += ctx->group)   // and quads compact inside each group
+        bisect_groups(L.c.data(), order.data() + k, std::min(ctx->group, n - k), 4);
     std::vector<float4> pos(n), par(n);
     std::vector<float2> sol(n);
     std::vector<double4> pos64(n), par64(n);
@@ -330,27 +345,31 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
         par64[k] = make_double4(L.svdw[i], L.rad[i], L.eps[i], L.heavy[i] ? 1.0 : 0.0);
         sol64[k] = make_double2(L.des[i], L.asa[i]);
     }
-    // bounding sphere of every group of ctx->group consecutive atoms (ligand
-    // frame), for the warp-cooperative kernel's candidate search
+    // bounding spheres (ligand frame) of every group of ctx->group and every
+    // quad of 4 consecutive atoms, for the warp kernels' candidate search
     const int G = ctx->group;
-    const int ngrp = (n + G - 1) / G;
-    std::vector<float4> grp(std::max(ngrp, 1));
-    for (int gi = 0; gi < ngrp; ++gi) {
-        const int a0 = gi * G, a1 = std::min(n, a0 + G);
-        double cen[3] = {0, 0, 0};
-        for (int k = a0; k < a1; ++k)
-            for (int a = 0; a < 3; ++a) cen[a] += L.c[3 * order[k] + a];
-        for (int a = 0; a < 3; ++a) cen[a] /= (a1 - a0);
-        double r2 = 0;
-        for (int k = a0; k < a1; ++k) {
-            double dd = 0;
-            for (int a = 0; a < 3; ++a) dd += (L.c[3 * order[k] + a] - cen[a]) * (L.c[3 * order[k] + a] - cen[a]);
-            r2 = std::max(r2, dd);
+    auto spheres = [&](int step) {
+        std::vector<float4> out(std::max((n + step - 1) / step, 1));
+        for (int gi = 0; gi * step < n; ++gi) {
+            const int a0 = gi * step, a1 = std::min(n, a0 + step);
+            double cen[3] = {0, 0, 0};
+            for (int k = a0; k < a1; ++k)
+                for (int a = 0; a < 3; ++a) cen[a] += L.c[3 * order[k] + a];
+            for (int a = 0; a < 3; ++a) cen[a] /= (a1 - a0);
+            double r2 = 0;
+            for (int k = a0; k < a1; ++k) {
+                double dd = 0;
+                for (int a = 0; a < 3; ++a) dd += (L.c[3 * order[k] + a] - cen[a]) * (L.c[3 * order[k] + a] - cen[a]);
+                r2 = std::max(r2, dd);
+            }
+            out[gi] = make_float4((float)cen[0], (float)cen[1], (float)cen[2], (float)(std::sqrt(r2) * (1.0 + 1e-6) + 1e-3));
         }
-        grp[gi] = make_float4((float)cen[0], (float)cen[1], (float)cen[2], (float)(std::sqrt(r2) * (1.0 + 1e-6) + 1e-3));
-    }
+        return out;
+    };
+    const std::vector<float4> grp = spheres(G), quad = spheres(4);
     cudaStream_t s = ctx->stream;
     LKG_CK(upload(cr.lgrp, grp, s), "upload ligand");
+    LKG_CK(upload(cr.lquad, quad, s), "upload ligand");
     LKG_CK(upload(cr.lpos, pos, s), "upload ligand");
     LKG_CK(upload(cr.lpar, par, s), "upload ligand");
     LKG_CK(upload(cr.lsolv, sol, s), "upload ligand");
@@ -364,6 +383,7 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
     d.lpos64 = cr.lpos64.as<double4>(); d.lpar64 = cr.lpar64.as<double4>(); d.lsolv64 = cr.lsolv64.as<double2>();
     d.lorig = cr.lorig.as<int>();
     d.lgrp = cr.lgrp.as<float4>();
+    d.lquad = cr.lquad.as<float4>();
     d.group = G;
     d.ntiles = std::max(1, (n + ctx->tile - 1) / ctx->tile);
     return set_ok();
@@ -466,7 +486,7 @@ static int set_rpar_tag_signs(lkg_ctx* ctx, ComplexRec& cr, const std::vector<in
         par[k].z = tagged ? -std::fabs(par[k].z) : std::fabs(par[k].z);
     }
     LKG_CK(cudaMemcpy(cr.rpar.p, par.data(), nr * sizeof(float4), cudaMemcpyHostToDevice), "receptor tags");
-    return 0;
+    return interleave_receptor(ctx, cr, nr);
 }
 
 int complex_set_ligand(lkg_ctx* ctx, int id, const MolIn& lig) {
@@ -681,6 +701,7 @@ int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, cons
     p.atom_elec = atom_e;
     p.atom_vdw = atom_v;
     p.pose_mask = pose_mask;
+    p.one = 1.0f;
     p.stage = ctx->stage_tma ? 1 : 0;
     for (int c : G.ic)   // restraints set after the groups were built (a plan made before)
         if (ctx->cx[c]->d.iface_words > G.iface_words)

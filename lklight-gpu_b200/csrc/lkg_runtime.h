@@ -79,9 +79,9 @@ struct MolIn {
 // device arrays of one complex; `d` points into them
 struct ComplexRec {
     int family = -1;
-    DBuf rpos, rpar, rsolv, rpos64, rpar64, rsolv64, rorig, cell_start;
+    DBuf rpos, rpar, rpk, rsolv, rpos64, rpar64, rsolv64, rorig, cell_start;
     DBuf rlb;   // distance lower bound of the receptor (ComplexDev::rlb)
-    DBuf lpos, lpar, lsolv, lpos64, lpar64, lsolv64, lorig, lgrp;
+    DBuf lpos, lpar, lsolv, lpos64, lpar64, lsolv64, lorig, lgrp, lquad;
     DBuf phi;
     DBuf rtag, ltag;   // interface tags (restraints / membrane), when set
     ComplexDev d{};
@@ -162,6 +162,9 @@ std::vector<float> receptor_distance_bound(const double* c, int n, int dims[3], 
 // (lkg_cells.cu), bit for bit the host build's
 int build_receptor_device(lkg_ctx* ctx, const MolIn& R, ComplexRec& cr, const float o[3], const int nc[3],
                           const float inv_e[3]);
+// both float4 of n atoms side by side, then an atom out of reach of everything
+// that adds nothing (ComplexDev::rpk; out: 2 (n + 1) float4)
+cudaError_t interleave_atoms(const float4* pos, const float4* par, int n, float4* out, cudaStream_t s);
 // replace the ligand of an existing complex (cuda_full_score)
 int complex_set_ligand(lkg_ctx* ctx, int id, const MolIn& lig);
 // a complex changed: descriptors to upload, captured graphs out of date

@@ -7,85 +7,87 @@
 // `p.tile` ligand atoms of one pose, split into groups of G consecutive
 // atoms (spatially compact: the ligand is ordered by recursive coordinate
 // bisection in groups of G) whose bounding sphere (centre, radius rho, in the
-// ligand frame) is computed on the host.  Per group:
+// ligand frame) is computed on the host, as is the sphere of every quad of 4
+// consecutive atoms.  Per group:
 //   1. lanes 0..G-1 transform their atom in f64 (kept as an f32 value plus
 //      the rounding residual), add the far-field term q * phi(x'), and park
-//      position and parameters in one of two slot sets in shared memory
-//      (the sets alternate between groups, so hits of one group can still be
-//      queued while the next group is set up);
+//      position and parameters in shared memory, two neighbouring atoms
+//      interleaved (a slot pair);
 //   2. the receptor rows (z, y cells of edge h) within 10 A + rho of the
 //      posed centre are enumerated 32 at a time (one per lane), trimmed in x
 //      to sub-cells of edge h / xsub, and turned into contiguous atom spans;
-//   3. 32 candidates at a time (lane -> span by a binary search over the
-//      warp's exclusive prefix of span lengths, coalesced float4 loads, the
-//      next chunk loaded while this one is tested) are tested against the G
-//      slot atoms (broadcast shared-memory reads), slot by slot; a ballot
-//      per slot appends that slot's hits (slot << 26 | receptor index) to
-//      the warp's ring buffer in lane order;
-//   4. while 32 or more hits are pending, each lane takes one and evaluates
-//      the pair terms with compensated distances and the exact d^2 <= 100
-//      test, accumulating in f64: the expensive math always runs on 32 lanes.
-// The warp's sums are reduced by shuffles into one partial per work unit;
-// the last unit of a pose sums the partials in tile order (deterministic:
-// the hit order is fixed by the algorithm, not by scheduling).
+//   3. 32 candidates at a time (coalesced float4 loads, the next chunk loaded
+//      while this one is tested) are tested against the spheres of the
+//      group's quads (10 A + the quad's radius) and join the candidate list
+//      of every quad they reach (a ballot and a popcount place them);
+//   4. a full list, and at the group's end every list, is scored densely:
+//      lane = (candidate, slot pair) with the slot pair in registers, every
+//      listed candidate against all 4 atoms of the quad, the exact d^2 <= 100
+//      test masking the sums.
+// The lists of 4 atoms hold 1.8-1.9 candidate tests per near pair (CPU model
+// at the batched workload's and a protein's atom densities; lists of 8 atoms
+// 2.4, of 16 atoms 3.3), so the pair terms are computed on every test, on
+// packed f32 pairs, without collecting the hits first.
+// A group's sums are reduced over the warp at the group's end and added in
+// group order: a pose's score does not depend on which warp took which part.
 #pragma once
+#include <type_traits>
+
 #include "lkg_score.cuh"
 
 namespace lkg {
 
 constexpr int WK_THREADS = 128;   // 4 independent warps per block
 
-// hit buffer: fewer than 64 pending hits (a batch of the plain kernel is 64
-// hits, two a lane) are moved to its front after each candidate chunk, so
-// the pending hits + the 32 x G hits of one chunk always fit
-template <int G> struct WRing { static constexpr int N = 32 * G + 64; };
+// candidates a quad's list holds: lists are scored when one holds more than
+// W_LIST - 64 (two chunks add at most 64)
+constexpr int W_LIST = 128;
 
-// resident blocks per SM the register budget is sized for: 64 registers a
-// thread for G = 8, 72 for G = 16 (measured 1.4 % faster than 80 at 6
-// blocks, 64 at 8 blocks 1.3 % slower), 80 for G = 32
-template <int G> struct WOcc { static constexpr int N = (G <= 8) ? 8 : (G == 16 ? 7 : 6); };
+// resident blocks per SM the register budget is sized for: 72 registers (a
+// few spills in the cold parts).  Sixteen complexes of 2,000 poses: 12.5 ms at
+// 5 blocks, 12.4 at 6, 12.1 at 7, 12.5 at 8.
+constexpr int WK_BLOCKS = 7;
 
 // per-warp desolvation state of the two slot sets (cpydock): the slot
 // atoms' f64 positions, their running minimum d^2 to non-excluded receptor
-// atoms (f64 bits; non-negative doubles order like their bit patterns) and
-// whether the ligand atom itself is excluded
+// atoms (f64 bits; non-negative doubles order like their bit patterns), and
+// the hits within 6.4 A that wait for it (slot << 26 | receptor index): fewer
+// than 32 wait when a step of 64 tests adds its own
 template <int G>
 struct WDes {
     double lx[2 * G], ly[2 * G], lz[2 * G];
     unsigned long long lmin[2 * G];
-    int lf[2 * G];
+    unsigned hit[96];
 };
 
 // interface words a warp collects in shared memory before merging them into
 // the pose's bits (larger sets go to HBM directly)
 constexpr int W_IBUF = 32;
-// hits of the packed pair path whose f32 d^2 lies within NEAR_BAND of the
-// 10 A cutoff wait here for the f64 decision (the scalar pair path), which
-// runs before their slot set is reused
-constexpr int W_DEFER = 64;
-// plain and interface kernels: candidates of the current group within its
-// sphere (x, y, z relative to the group centre, receptor index in w), tested
-// 32 at a time: a ring of 64, since fewer than 32 wait when a chunk of 32
-// more arrives
-constexpr int W_CQ = 64;
-struct WQueue {
-    float4 a[W_CQ];
+
+// two neighbouring ligand atoms, interleaved: every field is a packed f32
+// pair as the pair math takes it
+struct __align__(16) WPair {
+    float x[2], y[2], z[2];      // f64 position rounded to f32
+    float rx[2], ry[2], rz[2];   // and its rounding residual
+    float q[2], sv[2], r[2];     // charge, sqrt eps, radius
+    float h[2];                  // 0.75 for a heavy atom, else 0
 };
 
 template <int G>
 struct WSlots {
-    Rot rot;                    // pose of the current work unit
-    float4 lpos[2 * G];         // x, y, z (f32 part), q
-    float4 lres[2 * G];         // x, y, z residuals, sqrt eps
-    float4 ltest[2 * G];        // candidate test: -2 l', |l'|^2 - 100.01 (l' = l - group centre)
-    float2 lpar[2 * G];         // r, heavy
-    int ltag[2 * G];            // IFACE: restraint bit of the slot atom, -1 = none
-    unsigned* ibits;            // IFACE: interface bits of the current pose in HBM (null: none)
-    unsigned* iset;             // IFACE: where pairs set them: ibuf, or ibits when the pose has more words
-    unsigned ibuf[W_IBUF];      // IFACE: the unit's bits, merged into ibits once at the unit's end
-    unsigned hit[WRing<G>::N];  // (slot << 26) | receptor index, pending hits first
-    unsigned defer[W_DEFER];    // plain kernel: hits within f32 rounding of the cutoff, decided in f64 later
-    int ndefer;
+    Rot rot;                          // pose of the current work unit
+    WPair pair[G / 2];
+    float4 quad[(G + 3) / 4];         // candidate test of each quad's sphere: -2 c', R^2 - |c'|^2 (c' = c - group centre)
+    unsigned list[(G + 3) / 4][W_LIST + 16];   // receptor indices of each quad's candidates (and padding)
+    int first[(G + 3) / 4], cnt[(G + 3) / 4];   // the part of each list that is scored
+    float one[2];                     // 1, 1 (see w_d2)
+    int row[32];                      // per non-empty row of the current 32: first atom - the row's candidate offset
+    ComplexDev c;                     // descriptor of the current unit's complex
+    int ltag[G];                      // IFACE: restraint bit of the slot atom, -1 = none
+    float lf[G];                      // DESOLV: largest f32 d^2 of interest (-1: atom excluded)
+    unsigned* ibits;                  // IFACE: interface bits of the current pose in HBM (null: none)
+    unsigned* iset;                   // IFACE: where pairs set them: ibuf, or ibits when the pose has more words
+    unsigned ibuf[W_IBUF];            // IFACE: the unit's bits, merged into ibits once at the unit's end
 };
 
 // Staged candidates (the plain kernel's TMA variant, selected per context):
@@ -216,78 +218,6 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     return r;
 }
 
-// pair terms of one queued hit: the exact d^2 <= 100 test on the
-// compensated d^2, then the reference formulas (those of pair_fast, with
-// the LJ power taken as (rr^2 / d^2)^3) and the clash term selected instead
-// of branched on.  DESOLV: pairs that can lie within 6.4 A also update both
-// atoms' minimum distance in f64 (cpydock.rs:615-668), the ligand atom's in
-// its slot, the receptor atom's in the block's hash.  IFACE: pairs that can
-// lie within 3.9 A and involve a tagged atom are re-tested in f64 (the slot
-// position as f32 value + residual, ~2^-48 relative) and set the pose's
-// interface bits.
-template <int G, bool DESOLV, bool IFACE>
-__device__ __forceinline__ void w_pair(const ComplexDev& c, const WSlots<G>& W, WDes<G>* D, MinHash64* hash,
-                                       int* status, unsigned e, unsigned flags, unsigned* iset, double& elec,
-                                       double& vdw, int& np) {
-    const int l = (int)(e >> 26), k = (int)(e & 0x3ffffffu);
-    const float4 a = __ldg(c.rpos + k);
-    const float4 pr = __ldg(c.rpar + k);
-    const float4 lp = W.lpos[l], lr = W.lres[l];
-    const float2 lq = W.lpar[l];
-    const float dx = (lp.x - a.x) + lr.x, dy = (lp.y - a.y) + lr.y, dz = (lp.z - a.z) + lr.z;
-    const float d2 = dx * dx + dy * dy + dz * dz;
-    const bool in = fabsf(d2 - 100.f) < NEAR_BAND ? near_exact(c, k, lp.x, lr.x, lp.y, lr.y, lp.z, lr.z)
-                                                  : d2 <= 100.f;
-    if (!in) return;
-    ++np;
-    const float ir2 = rcp_approx(d2);
-    if (flags & F_ELEC) {
-        float ae = lp.w * a.w * ir2;
-        ae = fminf(fmaxf(ae, -ES_CAP_F), ES_CAP_F);
-        elec += (double)ae;
-    }
-    const float sv = lr.w * pr.x;
-    const float rr = lq.x + pr.y;
-    const float t = rr * rr * ir2;
-    const float p6 = t * t * t;
-    float vp = fminf(sv * p6 * (p6 - 2.f), 1.0f);
-    if (flags & F_CLASH) {   // uniform per complex: the other families skip the distance
-        const float d = d2 * rsqrt_approx(d2), dmin = 0.75f * rr;
-        const bool clash = lq.y != 0.f && pr.z != 0.f && d < dmin;
-        vp = clash ? vp + 6.f * (dmin - d) : vp;
-    }
-    vdw += (double)vp;
-    if (DESOLV && !D->lf[l] && pr.w == 0.f && d2 <= SOLV2_F * 1.001f) {
-        const double4 a64 = c.rpos64[k];
-        const double ex = D->lx[l] - a64.x, ey = D->ly[l] - a64.y, ez = D->lz[l] - a64.z;
-        const double d2d = ex * ex + ey * ey + ez * ez;
-        atomicMin(&D->lmin[l], (unsigned long long)__double_as_longlong(d2d));
-        if (d2d <= SOLV2_D && !hash->insert(k, d2d)) atomicOr(status, 1);
-    }
-    // tagged atoms carry the sign bit on their heavy flag (receptor: rpar.z,
-    // set with the restraints; ligand slot: lpar.y), which the != 0 tests
-    // above do not see: untagged pairs cost one test
-    if (IFACE && iset && d2 <= IFACE2_F && ((__float_as_uint(pr.z) | __float_as_uint(lq.y)) >> 31)) {
-        const int2 rt = __ldg(c.rtag + k);
-        const int lt = W.ltag[l];
-        {
-            const double4 a64 = c.rpos64[k];
-            double ex, ey, ez;
-            if (DESOLV) { ex = D->lx[l] - a64.x; ey = D->ly[l] - a64.y; ez = D->lz[l] - a64.z; }
-            else {
-                ex = ((double)lp.x + (double)lr.x) - a64.x;
-                ey = ((double)lp.y + (double)lr.y) - a64.y;
-                ez = ((double)lp.z + (double)lr.z) - a64.z;
-            }
-            if (ex * ex + ey * ey + ez * ez <= IFACE2_D) {
-                iface_set(iset, rt.x);
-                iface_set(iset, rt.y);
-                iface_set(iset, lt);
-            }
-        }
-    }
-}
-
 // Packed pairs of f32 (Blackwell's f32x2 FADD / FMUL / FFMA: one instruction
 // computes both lanes of the pair, each rounded as the scalar operation)
 struct F2 { unsigned long long v; };
@@ -306,105 +236,34 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     return r;
 }
 
-// two queued hits a lane (the plain kernel, no desolvation, no interface
-// bits): the pair terms of w_pair for hits e0 and e1 computed side by side
-// on packed f32 pairs, which halves the FP32 instructions of the pair math.
-// e1 counts only when v1 (a partial batch).  Same formulas as w_pair, per
-// hit; d^2 is summed as (dx^2 + dy^2) + dz^2 with the squares of (x, y)
-// taken as one packed pair, a difference of a few ulps from w_pair's
-// fused chain (the f64 decision near the cutoff sees through it).
-template <int G>
-__device__ __forceinline__ void w_pair2(const ComplexDev& c, WSlots<G>& W, unsigned e0, unsigned e1, bool v1,
-                                        unsigned flags, double& elec, double& vdw, int& np) {
-    const int l0 = (int)(e0 >> 26), k0 = (int)(e0 & 0x3ffffffu);
-    const int l1 = (int)(e1 >> 26), k1 = (int)(e1 & 0x3ffffffu);
-    const float4 a0 = __ldg(c.rpos + k0), a1 = __ldg(c.rpos + k1);
-    const float4 p0 = __ldg(c.rpar + k0), p1 = __ldg(c.rpar + k1);
-    const float4 lp0 = W.lpos[l0], lp1 = W.lpos[l1], lr0 = W.lres[l0], lr1 = W.lres[l1];
-    const float2 lq0 = W.lpar[l0], lq1 = W.lpar[l1];
-    // per hit: (x, y) as one packed pair (the float4s' aligned halves), z scalar
-    const F2 dxy0 = add2(sub2(f2(lp0.x, lp0.y), f2(a0.x, a0.y)), f2(lr0.x, lr0.y));
-    const F2 dxy1 = add2(sub2(f2(lp1.x, lp1.y), f2(a1.x, a1.y)), f2(lr1.x, lr1.y));
-    const float dz0 = (lp0.z - a0.z) + lr0.z, dz1 = (lp1.z - a1.z) + lr1.z;
-    float sx0, sy0, sx1, sy1;
-    f2_get(mul2(dxy0, dxy0), sx0, sy0);
-    f2_get(mul2(dxy1, dxy1), sx1, sy1);
-    const float d20 = fmaf(dz0, dz0, sy0 + sx0), d21 = fmaf(dz1, dz1, sy1 + sx1);
-    const F2 d2 = f2(d20, d21);
-    bool ok0 = d20 <= 100.f, ok1 = v1 && d21 <= 100.f;
-    // a hit within f32 rounding of the cutoff leaves this path for the
-    // deferred list (w_flush_deferred decides it in f64); were the list full
-    // (W_DEFER such hits before their slot set is reused) it keeps the f32
-    // decision
-    if (__builtin_expect(fabsf(d20 - 100.f) < NEAR_BAND, 0)) {
-        const int i = atomicAdd(&W.ndefer, 1);
-        if (i < W_DEFER) { W.defer[i] = e0; ok0 = false; }
-    }
-    if (__builtin_expect(v1 && fabsf(d21 - 100.f) < NEAR_BAND, 0)) {
-        const int i = atomicAdd(&W.ndefer, 1);
-        if (i < W_DEFER) { W.defer[i] = e1; ok1 = false; }
-    }
-    np += (int)ok0 + (int)ok1;
-    const F2 ir2 = f2(rcp_approx(d20), rcp_approx(d21));
-    if (flags & F_ELEC) {
-        float e0f, e1f;
-        f2_get(mul2(mul2(f2(lp0.w, lp1.w), f2(a0.w, a1.w)), ir2), e0f, e1f);
-        e0f = fminf(fmaxf(e0f, -ES_CAP_F), ES_CAP_F);
-        e1f = fminf(fmaxf(e1f, -ES_CAP_F), ES_CAP_F);
-        if (ok0) elec += (double)e0f;
-        if (ok1) elec += (double)e1f;
-    }
-    const F2 sv = mul2(f2(lr0.w, lr1.w), f2(p0.x, p1.x));
-    const F2 rr = add2(f2(lq0.x, lq1.x), f2(p0.y, p1.y));
-    const F2 t = mul2(mul2(rr, rr), ir2);
-    const F2 p6 = mul2(mul2(t, t), t);
-    float v0, vv1;
-    f2_get(mul2(mul2(sv, p6), sub2(p6, f2(2.f, 2.f))), v0, vv1);
-    v0 = fminf(v0, 1.0f);
-    vv1 = fminf(vv1, 1.0f);
-    if (flags & F_CLASH) {
-        const F2 d = mul2(d2, f2(rsqrt_approx(d20), rsqrt_approx(d21)));
-        const F2 dmin = mul2(f2(0.75f, 0.75f), rr);
-        float dd0, dd1, m0, m1, c0, c1;
-        f2_get(d, dd0, dd1);
-        f2_get(dmin, m0, m1);
-        f2_get(fma2(f2(6.f, 6.f), sub2(dmin, d), f2(v0, vv1)), c0, c1);
-        v0 = (lq0.y != 0.f && p0.z != 0.f && dd0 < m0) ? c0 : v0;
-        vv1 = (lq1.y != 0.f && p1.z != 0.f && dd1 < m1) ? c1 : vv1;
-    }
-    if (ok0) vdw += (double)v0;
-    if (ok1) vdw += (double)vv1;
+// one receptor atom, 32 bytes: (x, y, z, q), (sqrt eps, r, heavy, excluded);
+// atom nr is out of reach of everything (it pads the candidate lists)
+struct WAtom {
+    float4 a, p;
+};
+__device__ __forceinline__ WAtom w_atom(const float4* __restrict__ rpk, unsigned k) {
+    WAtom r;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.p.x), "=f"(r.p.y), "=f"(r.p.z), "=f"(r.p.w)
+        : "l"(rpk + 2 * (size_t)k));
+    return r;
 }
 
-// the deferred hits through the scalar pair path (which decides the cutoff
-// in f64 near it); out of line: it runs only when such hits exist
-template <int G>
-__device__ __noinline__ void w_flush_deferred(const ComplexDev& c, WSlots<G>& W, unsigned flags, double& elec,
-                                              double& vdw, int& np) {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();
-    const int n = min(W.ndefer, W_DEFER);
-    for (int i = lane; i < n; i += 32)
-        w_pair<G, false, false>(c, W, nullptr, nullptr, nullptr, W.defer[i], flags, nullptr, elec, vdw, np);
-    __syncwarp();
-    if (lane == 0) W.ndefer = 0;
-    __syncwarp();
+// the lane index, read once (a plain threadIdx.x & 31 is read again at every
+// use when registers are short)
+__device__ __forceinline__ int w_lane() {
+    unsigned l;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));
+    return (int)l;
 }
 
-// receptor atom of candidate kk of the current rows: the span is the last
-// row whose exclusive prefix is <= kk (empty rows never qualify ahead of the
-// non-empty row that follows them); far away when kk is past the end
-__device__ __forceinline__ void w_fetch(const ComplexDev& c, int st, int excl, int total, int kk, float4& a,
-                                        int& ridx) {
-    int rr = 0;
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-        const int v = __shfl_sync(0xffffffffu, excl, rr + s);
-        if (v <= kk) rr += s;
-    }
-    const int rst = __shfl_sync(0xffffffffu, st, rr), rex = __shfl_sync(0xffffffffu, excl, rr);
-    ridx = rst + (kk - rex);
-    a = kk < total ? __ldg(c.rpos + ridx) : make_float4(3e30f, 3e30f, 3e30f, 0.f);
+// the descriptor of a unit's complex into the warp's shared memory (its
+// fields are read all through a unit; from global memory each read waited)
+__device__ __forceinline__ void w_descriptor(ComplexDev* dst, const ComplexDev* src, int lane) {
+    static_assert(sizeof(ComplexDev) % 8 == 0, "copied in 8-byte words");
+    const unsigned long long* s = reinterpret_cast<const unsigned long long*>(src);
+    unsigned long long* d = reinterpret_cast<unsigned long long*>(dst);
+    for (int i = lane; i < (int)(sizeof(ComplexDev) / 8); i += 32) d[i] = __ldg(s + i);
 }
 
 constexpr unsigned long long W_NOMIN = 0x7fefffffffffffffull;   // largest finite double
@@ -420,48 +279,219 @@ __device__ __forceinline__ float w_receptor_bound(const ComplexDev& c, float x, 
 }
 
 
-// The warp's sums over its groups.
+// The warp's sums over its groups (cpydock: per lane; else per group, reduced).
 struct WAcc {
     double elec = 0.0, vdw = 0.0, solv = 0.0;
     int np = 0;
 };
 
-// Scores groups g_first, g_first + g_step, ... (< g_end) of one pose whose
-// rotation is in W.rot, into acc (per lane).  DESOLV also adds each slot
-// atom's g(min d^2) * des to acc.solv once its hits are all evaluated.
-template <int G, bool DESOLV, bool IFACE, bool STAGE = false>
-__device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes<G>* D, MinHash64* hash, int* status,
-                                         int g_first, int g_end, int g_step, WAcc& acc, WQueue* Q,
-                                         WStage* S = nullptr, bool far_sep = false) {
-    constexpr unsigned FULL = 0xffffffffu;
+// cpydock: the first n (<= 32) waiting hits, one a lane, update both atoms'
+// minimum distance in f64 (cpydock.rs:615-668), the ligand atom's in its slot,
+// the receptor atom's in the block's hash
+template <int G>
+__device__ __forceinline__ void w_minima(const ComplexDev& c, WDes<G>* D, MinHash64* hash, int* status, int first,
+                                         int n) {
     const int lane = threadIdx.x & 31;
+    if (lane >= n) return;
+    const unsigned e = D->hit[first + lane];
+    const int l = (int)(e >> 26), k = (int)(e & 0x3ffffffu);
+    const double4 a = c.rpos64[k];
+    const double ex = D->lx[l] - a.x, ey = D->ly[l] - a.y, ez = D->lz[l] - a.z;
+    const double d2 = ex * ex + ey * ey + ez * ez;
+    atomicMin(&D->lmin[l], (unsigned long long)__double_as_longlong(d2));
+    if (d2 <= SOLV2_D && !hash->insert(k, d2)) atomicOr(status, 1);
+}
+
+// d^2 of a receptor atom and both slots of a pair, from the compensated
+// differences (l - a) + residual.  CHAIN (cpydock and interface kernels): one
+// fused chain; else (dx^2 + dy^2) + dz^2 with the first sum rounded on its own
+// (`one` is 1, from memory: a plain packed add of two products is contracted)
+template <bool CHAIN>
+__device__ __forceinline__ F2 w_d2(const WPair& P, const WAtom& A, F2 one) {
+    const F2 dx = add2(f2(P.x[0] - A.a.x, P.x[1] - A.a.x), f2(P.rx[0], P.rx[1]));
+    const F2 dy = add2(f2(P.y[0] - A.a.y, P.y[1] - A.a.y), f2(P.ry[0], P.ry[1]));
+    const F2 dz = add2(f2(P.z[0] - A.a.z, P.z[1] - A.a.z), f2(P.rz[0], P.rz[1]));
+    return CHAIN ? fma2(dz, dz, fma2(dx, dx, mul2(dy, dy))) : fma2(dz, dz, fma2(mul2(dy, dy), one, mul2(dx, dx)));
+}
+
+// The listed pairs whose f32 d^2 lies within NEAR_BAND of the cutoff, which
+// w_dense leaves out: in or out as f64 decides.  Out of line: one test in some
+// ten thousand, so the lists of about one group in thirty are read again.
+template <int G, bool CHAIN>
+__device__ __noinline__ void w_band(const ComplexDev& c, const WSlots<G>& W, int lane, unsigned flags,
+                                    WAcc& r) {
+    for (int quad = 0; quad < (G + 3) / 4; ++quad)
+    for (int i = lane >> 1; i < W.cnt[quad]; i += 16) {
+        const WPair& P = W.pair[quad * 2 + (lane & 1)];
+        const unsigned k = W.list[quad][W.first[quad] + i];
+        const WAtom A{__ldg(c.rpk + 2 * (size_t)k), __ldg(c.rpk + 2 * (size_t)k + 1)};
+        float d20, d21;
+        f2_get(w_d2<CHAIN>(P, A, f2(W.one[0], W.one[1])), d20, d21);
+        for (int h = 0; h < 2; ++h) {
+            const float d2 = h ? d21 : d20;
+            if (!(fabsf(d2 - 100.f) < NEAR_BAND) || k >= (unsigned)c.nr ||
+                !near_exact(c, (int)k, P.x[h], P.rx[h], P.y[h], P.ry[h], P.z[h], P.rz[h]))
+                continue;
+            ++r.np;
+            const float ir2 = rcp_approx(d2);
+            if (flags & F_ELEC) r.elec += (double)fminf(fmaxf(P.q[h] * A.a.w * ir2, -ES_CAP_F), ES_CAP_F);
+            const float rr = P.r[h] + A.p.y, t = rr * rr * ir2, p6 = t * t * t;
+            float vp = fminf(P.sv[h] * A.p.x * p6 * (p6 - 2.f), 1.0f);
+            if (flags & F_CLASH)
+                vp = fmaf(6.f, fmaxf(P.h[h] * fabsf(A.p.z) * rr - d2 * rsqrt_approx(d2), 0.f), vp);
+            r.vdw += (double)vp;
+        }
+    }
+}
+
+// Scores n listed candidates (from list[first]) of quad `quad` densely: 16
+// candidates a step, lane = (candidate, slot pair), the slot pair in
+// registers, two steps side by side (two receptor atoms in flight, two
+// independent chains).  Per test the reference formulas on packed f32 pairs
+// (both slots of the pair).  off: the smallest |d^2 - 100| seen.  ELEC /
+// CLASH: the complex's terms.  The list is padded to a whole step.
+template <int G, bool DESOLV, bool IFACE, bool NP, bool ELEC, bool CLASH>
+__device__ __forceinline__ void w_dense(const ComplexDev& c, WSlots<G>& W, WDes<G>* D, MinHash64* hash, int* status,
+                                        unsigned* iset, int lane, int set, int quad, int first, int n, WAcc& acc,
+                                        float& off, int& nhit, int& old_hits) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int half = lane & 1;
+    const WPair P = W.pair[quad * 2 + half];
+    unsigned* const list = W.list[quad] + first;
+    const float4* rpk = c.rpk;
+    const F2 one = f2(W.one[0], W.one[1]);
+    const int slot0 = quad * 4 + half * 2;
+    // IFACE: a slot of the pair is tagged (untagged receptor atoms matter then)
+    const bool tagged = IFACE && iset && (W.ltag[slot0] >= 0 || W.ltag[slot0 + 1] >= 0);
+    float lf0 = 0.f, lf1 = 0.f;
+    if (DESOLV) { lf0 = W.lf[slot0]; lf1 = W.lf[slot0 + 1]; }
+    auto step = [&](const WAtom& A, unsigned k) {
+        const F2 d2 = w_d2<DESOLV || IFACE>(P, A, one);
+        float d20, d21, t0, t1;
+        f2_get(d2, d20, d21);
+        f2_get(sub2(d2, f2(100.f, 100.f)), t0, t1);
+        const F2 ir2 = f2(rcp_approx(d20), rcp_approx(d21));
+        float e0 = 0.f, e1 = 0.f, v0, v1;
+        if (ELEC) {
+            f2_get(mul2(f2(P.q[0] * A.a.w, P.q[1] * A.a.w), ir2), e0, e1);
+            e0 = fminf(fmaxf(e0, -ES_CAP_F), ES_CAP_F);
+            e1 = fminf(fmaxf(e1, -ES_CAP_F), ES_CAP_F);
+        }
+        const F2 sv = f2(P.sv[0] * A.p.x, P.sv[1] * A.p.x);
+        const F2 rr = f2(P.r[0] + A.p.y, P.r[1] + A.p.y);
+        const F2 t = mul2(mul2(rr, rr), ir2);
+        const F2 p6 = mul2(mul2(t, t), t);
+        f2_get(mul2(mul2(sv, p6), sub2(p6, f2(2.f, 2.f))), v0, v1);
+        v0 = fminf(v0, 1.0f);
+        v1 = fminf(v1, 1.0f);
+        if (CLASH) {
+            const float hz = fabsf(A.p.z);   // the sign marks a tagged atom
+            float g0, g1, m0, m1;
+            f2_get(mul2(d2, f2(rsqrt_approx(d20), rsqrt_approx(d21))), g0, g1);
+            f2_get(mul2(f2(P.h[0] * hz, P.h[1] * hz), rr), m0, m1);   // 0 unless both are heavy
+            v0 = fmaf(6.f, fmaxf(__fsub_rn(m0, g0), 0.f), v0);
+            v1 = fmaf(6.f, fmaxf(__fsub_rn(m1, g1), 0.f), v1);
+        }
+        // selected before the sums: a branch or a predicated f64 add cost more
+        const bool in0 = t0 <= -NEAR_BAND, in1 = t1 <= -NEAR_BAND;
+        if (ELEC) acc.elec = (acc.elec + (double)(in0 ? e0 : 0.f)) + (double)(in1 ? e1 : 0.f);
+        acc.vdw = (acc.vdw + (double)(in0 ? v0 : 0.f)) + (double)(in1 ? v1 : 0.f);
+        if (NP) acc.np += (int)in0 + (int)in1;
+        off = fminf(off, fminf(fabsf(t0), fabsf(t1)));
+        // tagged atoms carry the sign bit on their heavy flag (receptor) or a
+        // tag (slot): re-tested in f64 (the slot position as f32 value +
+        // residual, ~2^-48 relative), which sets the pose's interface bits
+        // (few atoms are tagged, so the tags are asked first: one pair in
+        // thirty is near enough, and then the whole warp would wait)
+        if (IFACE && ((__float_as_uint(A.p.z) >> 31) | (unsigned)tagged) && fminf(d20, d21) <= IFACE2_F) {
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const int lt = W.ltag[slot0 + h];
+                if (!iset || (h ? d21 : d20) > IFACE2_F || (lt < 0 && !(__float_as_uint(A.p.z) >> 31))) continue;
+                const double4 a64 = c.rpos64[k];
+                double ex, ey, ez;
+                if (DESOLV) {
+                    ex = D->lx[set + slot0 + h] - a64.x;
+                    ey = D->ly[set + slot0 + h] - a64.y;
+                    ez = D->lz[set + slot0 + h] - a64.z;
+                } else {
+                    const WPair& S = W.pair[quad * 2 + half];
+                    ex = ((double)S.x[h] + (double)S.rx[h]) - a64.x;
+                    ey = ((double)S.y[h] + (double)S.ry[h]) - a64.y;
+                    ez = ((double)S.z[h] + (double)S.rz[h]) - a64.z;
+                }
+                if (ex * ex + ey * ey + ez * ez <= IFACE2_D) {
+                    const int2 rt = __ldg(c.rtag + k);
+                    iface_set(iset, rt.x);
+                    iface_set(iset, rt.y);
+                    iface_set(iset, lt);
+                }
+            }
+        }
+        if (DESOLV) {
+            const bool s0 = d20 <= lf0 && A.p.w == 0.f, s1 = d21 <= lf1 && A.p.w == 0.f;
+            const unsigned b0 = __ballot_sync(FULL, s0), b1 = __ballot_sync(FULL, s1);
+            if (b0 | b1) {
+                const unsigned lt_mask = (1u << lane) - 1u;
+                const int n0 = __popc(b0);
+                if (s0) D->hit[nhit + __popc(b0 & lt_mask)] = ((unsigned)(set + slot0) << 26) | k;
+                if (s1) D->hit[nhit + n0 + __popc(b1 & lt_mask)] = ((unsigned)(set + slot0 + 1) << 26) | k;
+                nhit += n0 + __popc(b1);
+                __syncwarp();
+                int head = 0;
+                for (; nhit - head >= 32; head += 32) w_minima<G>(c, D, hash, status, head, 32);
+                if (head > 0) {   // the rest moves to the front
+                    const unsigned v = head + lane < nhit ? D->hit[head + lane] : 0u;
+                    __syncwarp();
+                    D->hit[lane] = v;
+                    nhit -= head;
+                    old_hits -= head;
+                    __syncwarp();
+                }
+            }
+        }
+    };
+    int i = 0;
+    for (; i + 16 < n; i += 32) {
+        const unsigned ka = list[i + (lane >> 1)], kb = list[i + 16 + (lane >> 1)];
+        const WAtom A = w_atom(rpk, ka), B = w_atom(rpk, kb);
+        step(A, ka);
+        step(B, kb);
+    }
+    if (i < n) {
+        const unsigned ka = list[i + (lane >> 1)];
+        step(w_atom(rpk, ka), ka);
+    }
+}
+
+// Scores groups g_first, g_first + g_step, ... (< g_end) of one pose whose
+// rotation is in W.rot.  Plain and interface kernels: after each group its
+// sums, reduced over the warp, are added to acc.elec (lanes 0-15: the
+// electrostatics, lanes 16-31: the vdW), so acc is the sum of the groups'
+// sums in order.  DESOLV: acc holds the lane's own sums, and each slot atom's
+// g(min d^2) * des is added to acc.solv once its hits are all evaluated.
+template <int G, bool DESOLV, bool IFACE, bool NP, bool STAGE = false>
+__device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes<G>* D, MinHash64* hash, int* status,
+                                         int lane, int g_first, int g_end, int g_step, WAcc& acc, WStage* S = nullptr,
+                                         bool far_sep = false) {
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int NQ = (G + 3) / 4;
     const unsigned lt_mask = (1u << lane) - 1u;
     const unsigned flags = c.flags;
     const int nl = c.nl;
     unsigned* const iset = IFACE ? W.iset : nullptr;   // set by the caller for the unit
-    // hits [head, tail) are pending; hits [head, prev_start) belong to the
-    // group before the previous one (whose slot set the next group reuses)
-    int head = 0, tail = 0, prev_start = 0;
+    int nhit = 0;                 // DESOLV: hits waiting for their minima
+    int old_hits = 0;             // DESOLV: the first of them, of groups before the previous one (may go below 0)
     int jdes0 = -1, jdes1 = -1;   // DESOLV: this lane's slot atom in set 0 / set 1
-    // the plain kernel evaluates 64 hits a batch (two a lane, packed f32
-    // pairs); the desolvation and interface kernels 32 (one a lane)
-    constexpr bool PAIR2 = !DESOLV && !IFACE;
-    constexpr int BATCH = PAIR2 ? 64 : 32;
-    auto drain_partial = [&]() {
-        const int n = tail - head;
-        if (n > lane) {
-            if (PAIR2)
-                w_pair2<G>(c, W, W.hit[head + lane], lane + 32 < n ? W.hit[head + 32 + lane] : W.hit[head + lane],
-                           lane + 32 < n, flags, acc.elec, acc.vdw, acc.np);
-            else
-                w_pair<G, DESOLV, IFACE>(c, W, D, hash, status, W.hit[head + lane], flags, iset, acc.elec, acc.vdw,
-                                         acc.np);
-        }
-        head = tail;
+    auto minima_rest = [&]() {
+        __syncwarp();
+        w_minima<G>(c, D, hash, status, 0, nhit);
+        nhit = 0;
+        __syncwarp();
     };
     auto finalize = [&](int set) {   // DESOLV: the slot set's minima are final
         const int j = set ? jdes1 : jdes0;
-        if (DESOLV && lane < G && j >= 0) {
+        if (lane < G && j >= 0) {
             const double2 ls = c.lsolv64[j];
             acc.solv += solv_term(__longlong_as_double((long long)D->lmin[set + lane]), ls.y) * ls.x;
         }
@@ -469,75 +499,97 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
     };
     int it = 0;
     for (int grp = g_first; grp < g_end; grp += g_step, ++it) {
-        const int set = (it & 1) * G;
-        // slot set `set` last served the group before the previous one, whose
-        // hits were queued before the previous group started: evaluate any
-        // still pending
-        if (prev_start > head) drain_partial();
-        if (PAIR2) {   // the deferred hits, before their slot set is reused
-            __syncwarp();
-            if (W.ndefer) w_flush_deferred<G>(c, W, flags, acc.elec, acc.vdw, acc.np);
-        }
-        prev_start = tail;
+        const int set = DESOLV ? (it & 1) * G : 0;
         __syncwarp();
-        finalize(set);
-        // 1. the group's ligand atoms
-        if (lane < G) {
+        if (DESOLV) {
+            // slot set `set` last served the group before the previous one,
+            // whose last hits may still wait
+            if (old_hits > 0) minima_rest();
+            old_hits = nhit;
+            finalize(set);
+        }
+        WAcc gsum;   // the group's near pairs and far field
+        // 1. the group's ligand atoms (lanes 0..G-1), the spheres of its quads
+        //    and its own (the lanes above; a second round with groups of 32)
+        float gx, gy, gz, R;
+        {
             const int j = grp * G + lane;
-            const bool valid = j < nl;
-            const float4 b4 = valid ? __ldg(c.lpos + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 lp4 = valid ? __ldg(c.lpar + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const bool atom = lane < G && j < nl;
+            // from the f64 base coordinates, as the reference transforms them
+            double4 b = make_double4(0.0, 0.0, 0.0, 0.0);
+            constexpr int Q0 = G < 32 ? G : 0;   // lane of the first quad
+            const int qi = grp * NQ + lane - Q0;
+            const bool quad = lane >= Q0 && lane < Q0 + NQ && qi * 4 < nl;
+            float rad = 0.f;
+            auto sphere = [&]() {
+                if (lane >= Q0 && lane <= Q0 + NQ) {
+                    const float4 s = lane == Q0 + NQ ? __ldg(c.lgrp + grp) : (quad ? __ldg(c.lquad + qi) : make_float4(0.f, 0.f, 0.f, 0.f));
+                    b = make_double4((double)s.x, (double)s.y, (double)s.z, 0.0);
+                    rad = SCAN_R + s.w;
+                }
+            };
+            if (atom) b = c.lpos64[j];
+            if (G < 32) sphere();
             double xd, yd, zd;
-            {   // from the f64 base coordinates, as the reference transforms them
-                const double4 b64 = valid ? c.lpos64[j] : make_double4(0.0, 0.0, 0.0, 0.0);
-                apply(W.rot, b64.x, b64.y, b64.z, xd, yd, zd);
-            }
+            apply(W.rot, b.x, b.y, b.z, xd, yd, zd);
             float x = (float)xd, y = (float)yd, z = (float)zd;
-            const float4 res = make_float4((float)(xd - (double)x), (float)(yd - (double)y),
-                                           (float)(zd - (double)z), lp4.x);
-            // far field with the reference's f64 interpolation (a per-atom
-            // cost; f32 here would add up over thousands of charged atoms)
-            // (the cpydock kernel takes it from k_far_poses instead when
-            // that pass ran: far_sep)
-            if (valid && (flags & F_FAR) && !(DESOLV && far_sep) && b4.w != 0.f)
-                acc.elec += c.lpos64[j].w * sample_phi(c, xd, yd, zd);
-            if (!valid) { x = y = z = 1e30f; }   // never within reach of a receptor atom
-            W.lpos[set + lane] = make_float4(x, y, z, b4.w);
-            W.lres[set + lane] = res;
-            const int ltg = (IFACE && valid && c.ltag) ? __ldg(c.ltag + j) : -1;
-            W.lpar[set + lane] = make_float2(lp4.y, ltg >= 0 ? -lp4.z : lp4.z);   // -0 or -1 when tagged
-            if (IFACE) W.ltag[set + lane] = ltg;
-            if (DESOLV) {
-                D->lx[set + lane] = xd; D->ly[set + lane] = yd; D->lz[set + lane] = zd;
-                D->lmin[set + lane] = W_NOMIN;
-                D->lf[set + lane] = lp4.w != 0.f;
-                if (set) jdes1 = valid ? j : -1; else jdes0 = valid ? j : -1;
+            if (lane < G) {
+                const float4 lp4 = atom ? __ldg(c.lpar + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float q = (float)b.w;
+                WPair& P = W.pair[lane >> 1];
+                const int h = lane & 1;
+                P.rx[h] = (float)(xd - (double)x);
+                P.ry[h] = (float)(yd - (double)y);
+                P.rz[h] = (float)(zd - (double)z);
+                P.x[h] = atom ? x : 1e30f;   // never within reach of a receptor atom
+                P.y[h] = atom ? y : 1e30f;
+                P.z[h] = atom ? z : 1e30f;
+                P.q[h] = q; P.sv[h] = lp4.x; P.r[h] = lp4.y;
+                P.h[h] = lp4.z != 0.f ? 0.75f : 0.f;
+                if (IFACE) W.ltag[lane] = (atom && c.ltag) ? __ldg(c.ltag + j) : -1;
+                if (DESOLV) {
+                    D->lx[set + lane] = xd; D->ly[set + lane] = yd; D->lz[set + lane] = zd;
+                    D->lmin[set + lane] = W_NOMIN;
+                    W.lf[lane] = lp4.w != 0.f ? -1.f : SOLV2_F * 1.001f;
+                    if (set) jdes1 = atom ? j : -1; else jdes0 = atom ? j : -1;
+                }
+                // far field with the reference's f64 interpolation (a per-atom
+                // cost; f32 here would add up over thousands of charged atoms)
+                // (the cpydock kernel takes it from k_far_poses instead when
+                // that pass ran: far_sep)
+                if (atom && (flags & F_FAR) && !(DESOLV && far_sep) && q != 0.f)
+                    gsum.elec = b.w * sample_phi(c, xd, yd, zd);
+            }
+            if (G == 32) {
+                sphere();
+                apply(W.rot, b.x, b.y, b.z, xd, yd, zd);
+                x = (float)xd; y = (float)yd; z = (float)zd;
+            }
+            gx = __shfl_sync(FULL, x, Q0 + NQ);
+            gy = __shfl_sync(FULL, y, Q0 + NQ);
+            gz = __shfl_sync(FULL, z, Q0 + NQ);
+            R = __shfl_sync(FULL, rad, Q0 + NQ);
+            if (lane >= Q0 && lane < Q0 + NQ) {
+                // |a' - c'|^2 <= R^2 as |a'|^2 - 2 a'.c' <= R^2 - |c'|^2 in the
+                // group frame (|a'| <= ~20 A: rounding ~1e-4, far inside the
+                // 0.02 A^2 that SCAN_R leaves); a quad past the ligand never passes
+                const float lx = (float)(xd - (double)gx), ly = (float)(yd - (double)gy), lz = (float)(zd - (double)gz);
+                W.quad[lane - Q0] = quad ? make_float4(-2.f * lx, -2.f * ly, -2.f * lz,
+                                                       rad * rad - (lx * lx + ly * ly + lz * lz))
+                                         : make_float4(0.f, 0.f, 0.f, -3e30f);
             }
         }
         // 2. receptor rows within reach of the group sphere
-        const float4 gs = __ldg(c.lgrp + grp);
-        double cxd, cyd, czd;
-        apply(W.rot, (double)gs.x, (double)gs.y, (double)gs.z, cxd, cyd, czd);
-        const float gx = (float)cxd, gy = (float)cyd, gz = (float)czd;
-        if (lane < G) {
-            // candidate test |a' - l'|^2 <= 100.01 as |a'|^2 - 2 a'.l' +
-            // |l'|^2 in the group frame (|a'| <= ~20 A: rounding ~1e-4,
-            // far inside the 0.01 margin); invalid slots never pass
-            const float4 lp = W.lpos[set + lane];
-            const float lx = lp.x - gx, ly = lp.y - gy, lz = lp.z - gz;
-            const bool far_slot = !(lp.x < 1e29f);
-            W.ltest[set + lane] = far_slot ? make_float4(0.f, 0.f, 0.f, 3e30f)
-                                           : make_float4(-2.f * lx, -2.f * ly, -2.f * lz,
-                                                         lx * lx + ly * ly + lz * lz - 100.01f);
-        }
-        __syncwarp();
-        const float R = SCAN_R + gs.w, R2 = R * R;
+        const float R2 = R * R;
         // cpydock kernel: no receptor atom within R of the centre, so the
         // group has no candidate and its rows are not enumerated (most groups
         // of a large ligand at the interface: with a 12,000-atom ligand on a
         // 101,000-atom receptor the step is 4.5 % faster; the plain kernel,
         // whose ligands are smaller, measured 1 % slower with the test)
-        if (DESOLV && c.rlb && R < c.rlb_m && w_receptor_bound(c, gx, gy, gz) > R) continue;
+        if (DESOLV && c.rlb && R < c.rlb_m && w_receptor_bound(c, gx, gy, gz) > R) {
+            acc.elec += gsum.elec;
+            continue;
+        }
         const int cz0 = max(0, (int)floorf((gz - R - c.oz) * c.inv_h));
         const int cz1 = min(c.ncz - 1, (int)floorf((gz + R - c.oz) * c.inv_h));
         const int cy0 = max(0, (int)floorf((gy - R - c.oy) * c.inv_h));
@@ -545,139 +597,107 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
         const int nyr = cy1 - cy0 + 1, nzr = cz1 - cz0 + 1;
         const int nbox = (nyr > 0 && nzr > 0) ? nyr * nzr : 0;
         const float inv_nyr = 1.0f / (float)max(nyr, 1);
-        const unsigned enc_set = (unsigned)set << 26;
-        // 3. queued candidates, 32 a time: each lane tests its candidate
-        //    (relative to the group centre) against the group's slots and
-        //    appends its hits
-        auto test_chunk = [&](const float ax, const float ay, const float az, const int ridx) {
-            const float aa = ax * ax + ay * ay + az * az;
-            // the lane's candidate against every slot: a bit per hit
-            unsigned m = 0;
+        int cnt[NQ];   // list lengths
 #pragma unroll
-            for (int l = 0; l < G; ++l) {
-                const float4 t = W.ltest[set + l];
-                // |a'|^2 - 2 a'.l' <= -(|l'|^2 - 100.01): three FMAs, the
-                // slot's constant on the right (invalid slots: -3e30)
-                const float q = fmaf(ax, t.x, fmaf(ay, t.y, fmaf(az, t.z, aa)));
-                m |= (q <= -t.w ? 1u : 0u) << l;
-            }
-            // lane-major append: each lane writes its hits (slot order)
-            // at the warp's exclusive prefix of the hit counts
-            const int nh = __popc(m);
-            int inc = nh;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(FULL, inc, o);
-                if (lane >= o) inc += v;
-            }
-            const int chunk_hits = __shfl_sync(FULL, inc, 31);
-            if (chunk_hits == 0) return;
-            unsigned* dst = W.hit + tail + (inc - nh);
-            const unsigned enc = (unsigned)ridx | enc_set;
-#pragma unroll
-            for (int l = 0; l < G; ++l)
-                if (m & (1u << l)) *dst++ = enc + ((unsigned)l << 26);
-            tail += chunk_hits;
-            __syncwarp();
-            // 4. full batches
-            while (tail - head >= BATCH) {
-                if (PAIR2)
-                    w_pair2<G>(c, W, W.hit[head + lane], W.hit[head + 32 + lane], true, flags, acc.elec,
-                               acc.vdw, acc.np);
-                else
-                    w_pair<G, DESOLV, IFACE>(c, W, D, hash, status, W.hit[head + lane], flags, iset, acc.elec,
-                                             acc.vdw, acc.np);
-                head += BATCH;
-            }
-            // keep the buffer linear: the < BATCH pending hits move to its front
-            if (head > 0) {
-                const int rem = tail - head;
-                const unsigned v = lane < rem ? W.hit[head + lane] : 0u;
-                const unsigned v2 = (PAIR2 && lane + 32 < rem) ? W.hit[head + 32 + lane] : 0u;
-                __syncwarp();
-                if (lane < rem) W.hit[lane] = v;
-                if (PAIR2 && lane + 32 < rem) W.hit[32 + lane] = v2;
-                __syncwarp();
-                prev_start = max(prev_start - head, 0);
-                tail = rem;
-                head = 0;
-            }
-        };
-        // a candidate farther than R from the group centre is more than 10 A
-        // from every slot atom (|l'| <= rho).  The plain and interface
-        // kernels queue only the candidates within R (the row spans' corners
-        // outside the sphere, about 40 % of the candidates with 6 A cells,
-        // then cost no slot tests); the cpydock kernel, short of shared
-        // memory and L1, tests whole chunks and skips those with none within R
-        int q_head = 0, q_tail = 0;
+        for (int s = 0; s < NQ; ++s) cnt[s] = 0;
+        // 3. 32 candidates (relative to the group centre): listed for every
+        //    quad whose sphere they are in
         auto chunk = [&](const float4 a, const int ridx) {
             const float ax = a.x - gx, ay = a.y - gy, az = a.z - gz;
-            const bool in = ax * ax + ay * ay + az * az <= R2;
-            if (DESOLV) {
-                if (__any_sync(FULL, in)) test_chunk(ax, ay, az, ridx);
-                return;
-            }
-            const unsigned b = __ballot_sync(FULL, in);
-            if (in)
-                Q->a[(q_tail + __popc(b & lt_mask)) & (W_CQ - 1)] = make_float4(ax, ay, az, __int_as_float(ridx));
-            q_tail += __popc(b);
-            if (q_tail - q_head >= 32) {
-                __syncwarp();
-                const float4 q = Q->a[(q_head + lane) & (W_CQ - 1)];
-                q_head += 32;
-                test_chunk(q.x, q.y, q.z, __float_as_int(q.w));
+            const float aa = ax * ax + ay * ay + az * az;
+#pragma unroll
+            for (int s = 0; s < NQ; ++s) {
+                const float4 t = W.quad[s];
+                const bool in = fmaf(ax, t.x, fmaf(ay, t.y, fmaf(az, t.z, aa))) <= t.w;
+                const unsigned b = __ballot_sync(FULL, in);
+                if (in) W.list[s][cnt[s] + __popc(b & lt_mask)] = (unsigned)ridx;
+                cnt[s] += __popc(b);
             }
         };
-        for (int r0 = 0; r0 < nbox; r0 += 32) {
-            const int r = r0 + lane;
-            int st = 0, len = 0;
-            if (r < nbox) {
-                // r = zz * nyr + yy; (r + 0.5) / nyr is at least 0.5 / nyr
-                // away from an integer, far above the f32 rounding error
-                const int zz = (int)(((float)r + 0.5f) * inv_nyr), yy = r - zz * nyr;
-                const int cz = cz0 + zz, cy = cy0 + yy;
-                const float zlo = c.oz + cz * c.h, ylo = c.oy + cy * c.h;
-                const float dzm = fmaxf(0.f, fmaxf(zlo - gz, gz - (zlo + c.h)));
-                const float dym = fmaxf(0.f, fmaxf(ylo - gy, gy - (ylo + c.h)));
-                const float rem = R2 - dzm * dzm - dym * dym;
-                if (rem >= 0.f) {
-                    const float wx = sqrtf(rem);
-                    const int cx0 = max(0, (int)floorf((gx - wx - c.ox) * c.inv_hx));
-                    const int cx1 = min(c.ncx - 1, (int)floorf((gx + wx - c.ox) * c.inv_hx));
-                    if (cx0 <= cx1) {
-                        const int row = (cz * c.ncy + cy) * c.ncx;
-                        st = __ldg(c.cell_start + row + cx0);
-                        len = __ldg(c.cell_start + row + cx1 + 1) - st;
-                    }
-                }
-            }
-            int inc = len;   // inclusive prefix of the span lengths
+        auto full = [&]() {   // two more chunks may not fit
+            int m = cnt[0];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(FULL, inc, o);
-                if (lane >= o) inc += v;
-            }
-            const int total = __shfl_sync(FULL, inc, 31);
-            const int excl = inc - len;
-            if (!STAGE) {
-                // the next chunk's receptor atoms are fetched (through L1)
-                // while the current one is tested
-                float4 an = make_float4(3e30f, 3e30f, 3e30f, 0.f);
-                int rn = 0;
-                if (total > 0) w_fetch(c, st, excl, total, lane, an, rn);
-                for (int k0 = 0; k0 < total; k0 += 32) {
-                    const float4 a = an;
-                    const int ridx = rn;
-                    if (k0 + 32 < total) w_fetch(c, st, excl, total, k0 + 32 + lane, an, rn);
-                    chunk(a, ridx);
+            for (int s = 1; s < NQ; ++s) m = max(m, cnt[s]);
+            return m > W_LIST - 64;
+        };
+        const float4 far_away = make_float4(3e30f, 3e30f, 3e30f, 0.f);
+        int r0 = -32;                                     // the current 32 rows
+        int st = 0, len = 0, excl = 0, total = 0;         // this lane's row: first atom, atoms, candidates before it; all rows' candidates
+        int k0 = 0, rows = 0;                             // next candidate, rows that start before it
+        bool more = true;
+        // candidate kk belongs to the last non-empty row that starts at or
+        // before it: the starts within a chunk of 32 as a bit mask, the rows
+        // before the chunk counted in `rows`
+        auto locate = [&](int kc) {   // receptor index of candidate kc + lane (chunks in order)
+            const unsigned d = (unsigned)(excl - kc);
+            const unsigned m = __reduce_or_sync(FULL, (len > 0 && d < 32u) ? 1u << d : 0u);
+            const int ord = rows + __popc(m & (lt_mask | (1u << lane))) - 1;
+            rows += __popc(m);
+            return W.row[ord] + kc + lane;
+        };
+        do {
+            while (!full()) {
+                if (k0 >= total) {
+                    r0 += 32;
+                    if (r0 >= nbox) { more = false; break; }
+                    const int r = r0 + lane;
+                    st = len = 0;
+                    if (r < nbox) {
+                        // r = zz * nyr + yy; (r + 0.5) / nyr is at least 0.5 / nyr
+                        // away from an integer, far above the f32 rounding error
+                        const int zz = (int)(((float)r + 0.5f) * inv_nyr), yy = r - zz * nyr;
+                        const int cz = cz0 + zz, cy = cy0 + yy;
+                        const float zlo = c.oz + cz * c.h, ylo = c.oy + cy * c.h;
+                        const float dzm = fmaxf(0.f, fmaxf(zlo - gz, gz - (zlo + c.h)));
+                        const float dym = fmaxf(0.f, fmaxf(ylo - gy, gy - (ylo + c.h)));
+                        const float rem = R2 - dzm * dzm - dym * dym;
+                        if (rem >= 0.f) {
+                            const float wx = sqrtf(rem);
+                            const int cx0 = max(0, (int)floorf((gx - wx - c.ox) * c.inv_hx));
+                            const int cx1 = min(c.ncx - 1, (int)floorf((gx + wx - c.ox) * c.inv_hx));
+                            if (cx0 <= cx1) {
+                                const int row = (cz * c.ncy + cy) * c.ncx;
+                                st = __ldg(c.cell_start + row + cx0);
+                                len = __ldg(c.cell_start + row + cx1 + 1) - st;
+                            }
+                        }
+                    }
+                    int inc = len;   // inclusive prefix of the span lengths
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int v = __shfl_up_sync(FULL, inc, o);
+                        if (lane >= o) inc += v;
+                    }
+                    total = __shfl_sync(FULL, inc, 31);
+                    excl = inc - len;
+                    k0 = rows = 0;
+                    const unsigned ne = __ballot_sync(FULL, len > 0);
+                    __syncwarp();
+                    if (len > 0) W.row[__popc(ne & lt_mask)] = st - excl;
+                    __syncwarp();
+                    if (total == 0) continue;
                 }
-            } else {
-                // windows of STAGE_WIN candidates: every row span's part of
-                // the window is bulk-copied into shared memory by its lane
-                const uint32_t bar = w_smem_u32(&S->bar);
-                for (int w0 = 0; w0 < total; w0 += STAGE_WIN) {
-                    const int wn = min(STAGE_WIN, total - w0);
-                    const int lo = max(excl, w0), hi = min(excl + len, w0 + wn);
+                if (!STAGE) {
+                    // two chunks in flight, through L1; from rpk, whose lines
+                    // the scoring reads again
+                    const bool two = k0 + 32 < total;
+                    const int ra = locate(k0);
+                    const float4 a = k0 + lane < total ? __ldg(c.rpk + 2 * (size_t)ra) : far_away;
+                    if (two) {
+                        const int rb = locate(k0 + 32);
+                        const float4 b = k0 + 32 + lane < total ? __ldg(c.rpk + 2 * (size_t)rb) : far_away;
+                        chunk(a, ra);
+                        chunk(b, rb);
+                    } else {
+                        chunk(a, ra);
+                    }
+                    k0 += 64;
+                } else {
+                    // windows of STAGE_WIN candidates: every row span's part of
+                    // the window is bulk-copied into shared memory by its lane
+                    const uint32_t bar = w_smem_u32(&S->bar);
+                    const int wn = min(STAGE_WIN, total - k0);
+                    const int lo = max(excl, k0), hi = min(excl + len, k0 + wn);
                     __syncwarp();   // the previous window is read
                     if (lane == 0)
                         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
@@ -687,7 +707,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         asm volatile(
                             "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                            :: "r"(w_smem_u32(S->a + (lo - w0))),
+                            :: "r"(w_smem_u32(S->a + (lo - k0))),
                                "l"(reinterpret_cast<uint64_t>(c.rpos + st + (lo - excl))),
                                "r"((uint32_t)(hi - lo) * 16u), "r"(bar) : "memory");
                     }
@@ -700,50 +720,85 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
                     __syncwarp();
                     if (lane == 0) S->phase = ph ^ 1u;
                     __syncwarp();
-                    for (int k0 = w0; k0 < w0 + wn; k0 += 32) {
-                        const int kk = k0 + lane;
-                        int rr = 0;
-#pragma unroll
-                        for (int sft = 16; sft > 0; sft >>= 1) {
-                            const int v = __shfl_sync(FULL, excl, rr + sft);
-                            if (v <= kk) rr += sft;
-                        }
-                        const int ridx = __shfl_sync(FULL, st, rr) + (kk - __shfl_sync(FULL, excl, rr));
-                        const float4 a = kk < w0 + wn ? S->a[kk - w0] : make_float4(3e30f, 3e30f, 3e30f, 0.f);
-                        chunk(a, ridx);
+                    for (int kc = 0; kc < wn; kc += 32) {
+                        const int ridx = locate(k0 + kc);
+                        chunk(kc + lane < wn ? S->a[kc + lane] : far_away, ridx);
                     }
+                    k0 += STAGE_WIN;
                 }
             }
-        }
-        // the queue's remainder (the lanes past it test a far candidate)
-        if (!DESOLV && q_tail > q_head) {
+            // 4. the lists, scored: whole steps of 16 of the longer ones while
+            //    the group goes on (the end of a list first, so its rest stays
+            //    at the front), all at its end
+            float off = 1e30f;
+#pragma unroll
+            for (int s = 0; s < NQ; ++s) {
+                // the length to score, and padding past the list's end
+                const int m = !more ? cnt[s] : (cnt[s] >= 32 ? cnt[s] & ~15 : 0);
+                if (lane < 16) W.list[s][cnt[s] + lane] = (unsigned)c.nr;
+                if (lane == s) { W.cnt[s] = m; W.first[s] = cnt[s] - m; }
+                cnt[s] -= m;
+            }
             __syncwarp();
-            const int n = q_tail - q_head;
-            const float4 q = lane < n ? Q->a[(q_head + lane) & (W_CQ - 1)] : make_float4(3e30f, 3e30f, 3e30f, 0.f);
-            test_chunk(q.x, q.y, q.z, __float_as_int(q.w));
+            auto lists = [&](auto elec, auto clash) {
+#pragma unroll 1
+                for (int s = 0; s < NQ; ++s)
+                    w_dense<G, DESOLV, IFACE, NP, decltype(elec)::value, decltype(clash)::value>(
+                        c, W, D, hash, status, iset, lane, set, s, W.first[s], W.cnt[s], gsum, off, nhit, old_hits);
+            };
+            using T = std::true_type;
+            using F = std::false_type;
+            if (DESOLV) {
+                if (flags & F_ELEC) lists(T(), F()); else lists(F(), F());
+            } else switch (flags & (F_ELEC | F_CLASH)) {
+                case F_ELEC | F_CLASH: lists(T(), T()); break;
+                case F_ELEC: lists(T(), F()); break;
+                case F_CLASH: lists(F(), T()); break;
+                default: lists(F(), F()); break;
+            }
+            if (__any_sync(FULL, off < NEAR_BAND)) {
+                WAcc r;
+                w_band<G, DESOLV || IFACE>(c, W, lane, flags, r);
+                gsum.elec += r.elec;
+                gsum.vdw += r.vdw;
+                if (NP) gsum.np += r.np;
+            }
+            __syncwarp();
+        } while (more);
+        if (NP) acc.np += gsum.np;
+        if (DESOLV) {
+            acc.elec += gsum.elec;
+            acc.vdw += gsum.vdw;
+        } else {
+            // the group's sums over the warp: electrostatics in lanes 0-15,
+            // vdW in lanes 16-31
+            const bool hi = lane >= 16;
+            double keep = hi ? gsum.vdw : gsum.elec;
+            keep += __shfl_xor_sync(FULL, hi ? gsum.elec : gsum.vdw, 16);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) keep += __shfl_xor_sync(FULL, keep, o);
+            acc.elec += keep;
         }
     }
-    __syncwarp();
-    drain_partial();
-    __syncwarp();
-    if (PAIR2 && W.ndefer) w_flush_deferred<G>(c, W, flags, acc.elec, acc.vdw, acc.np);
-    finalize(0);
-    finalize(G);
+    if (DESOLV) {
+        minima_rest();
+        finalize(0);
+        finalize(G);
+    }
 }
 
 // STAGE: the candidates reach shared memory by bulk copies (WStage) instead
 // of L1 loads (selected per context; the measured alternative)
-template <int G, bool IFACE, bool STAGE = false>
-__global__ void __launch_bounds__(WK_THREADS, WOcc<G>::N) k_score_warp(LaunchParams p) {
+// NP: near pairs are counted (launches with parts)
+template <int G, bool IFACE, bool NP, bool STAGE = false>
+__global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchParams p) {
     static_assert(G == 4 || G == 8 || G == 16 || G == 32, "group size");
     static_assert(!(STAGE && IFACE), "the staged variant is the plain kernel's");
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char wk_smem[];
-    const int lane = threadIdx.x & 31;
+    const int lane = w_lane();
     WSlots<G>& W = reinterpret_cast<WSlots<G>*>(wk_smem)[threadIdx.x >> 5];
-    WQueue* Q = reinterpret_cast<WQueue*>(wk_smem + (WK_THREADS / 32) * sizeof(WSlots<G>)) + (threadIdx.x >> 5);
-    WStage* S = STAGE ? reinterpret_cast<WStage*>(wk_smem + (WK_THREADS / 32) * (sizeof(WSlots<G>) + sizeof(WQueue))) +
-                            (threadIdx.x >> 5)
+    WStage* S = STAGE ? reinterpret_cast<WStage*>(wk_smem + (WK_THREADS / 32) * sizeof(WSlots<G>)) + (threadIdx.x >> 5)
                       : nullptr;
     if (STAGE) {
         if (lane == 0) {
@@ -754,15 +809,23 @@ __global__ void __launch_bounds__(WK_THREADS, WOcc<G>::N) k_score_warp(LaunchPar
         __syncwarp();
     }
     if (IFACE) W.ibuf[lane] = 0u;
-    if (lane == 0) W.ndefer = 0;
+    if (lane < 2) W.one[lane] = p.one;
     __syncwarp();
+    int cur = -1;   // complex whose descriptor W.c holds
     for (;;) {
         unsigned long long wq = 0;
         if (lane == 0) wq = atomicAdd(p.work_counter, 1ull);
         const long long w = (long long)__shfl_sync(FULL, wq, 0);
         if (w >= p.total_work) break;
         const int b = find_item(p.item_work0, p.n_items, w);
-        const ComplexDev& c = p.cx[__ldg(p.item_complex + b)];
+        const int cid = __ldg(p.item_complex + b);
+        if (cid != cur) {
+            __syncwarp();
+            w_descriptor(&W.c, p.cx + cid, lane);
+            cur = cid;
+            __syncwarp();
+        }
+        const ComplexDev& c = W.c;
         const long long local = w - __ldg(p.item_work0 + b);
         const int ntiles = c.ntiles;
         const int pose = (int)(local / ntiles), tile = (int)(local % ntiles);
@@ -778,26 +841,35 @@ __global__ void __launch_bounds__(WK_THREADS, WOcc<G>::N) k_score_warp(LaunchPar
         const int gpt = p.tile / G;
         const int g0 = tile * gpt, g1 = min(g0 + gpt, (c.nl + G - 1) / G);
         WAcc acc;
-        w_groups<G, false, IFACE, STAGE>(c, W, nullptr, nullptr, p.status, g0, g1, 1, acc, Q, S);
-        if (IFACE && W.ibits) {
-            w_iface_flush(W, c);
-            __threadfence();   // interface bits before the unit is published
+        w_groups<G, false, IFACE, NP, STAGE>(c, W, nullptr, nullptr, p.status, lane, g0, g1, 1, acc, S);
+        if (IFACE && W.ibits) w_iface_flush(W, c);
+        // partial of work unit w; the pose's units are w - tile .. w - tile + ntiles - 1
+        double* part = p.partials + (size_t)w * 4;
+        if (lane == 0) part[0] = acc.elec;
+        if (lane == 16) part[1] = acc.elec;   // the vdW half
+        if (NP) {
+            const int npl = (int)__reduce_add_sync(FULL, (unsigned)acc.np);
+            if (lane == 0) part[3] = (double)npl;
         }
-        const double elec = warp_sum(acc.elec), vdw = warp_sum(acc.vdw);
-        const long long npl = warp_sum((long long)acc.np);
-        if (lane == 0) {
-            // partial of work unit w; the pose's units are w - tile .. w - tile + ntiles - 1
-            double* part = p.partials + (size_t)w * 4;
-            part[0] = elec; part[1] = vdw; part[2] = 0.0; part[3] = (double)npl;
+        __threadfence();   // partial (and interface bits) before the unit is published
+        __syncwarp();
+        int done = 0;
+        if (lane == 0) done = atomicAdd(p.pose_counter + g, 1);
+        done = __shfl_sync(FULL, done, 0);
+        if (done == ntiles - 1) {
             __threadfence();
-            const int done = atomicAdd(p.pose_counter + g, 1);
-            if (done == ntiles - 1) {
-                __threadfence();
-                double e = 0.0, vv = 0.0, nps = 0.0;
-                const double* pp = p.partials + (size_t)(w - tile) * 4;
-                for (int t = 0; t < ntiles; ++t) {
-                    e += __ldcg(pp + 4 * t); vv += __ldcg(pp + 4 * t + 1); nps += __ldcg(pp + 4 * t + 3);
-                }
+            // lane i sums tiles i, i + 32, ..., then a fixed tree
+            double e = 0.0, vv = 0.0, nps = 0.0;
+            const double* pp = p.partials + (size_t)(w - tile) * 4;
+            for (int t = lane; t < ntiles; t += 32) {
+                e += __ldcg(pp + 4 * t);
+                vv += __ldcg(pp + 4 * t + 1);
+                if (NP) nps += __ldcg(pp + 4 * t + 3);
+            }
+            e = warp_sum(e);
+            vv = warp_sum(vv);
+            if (NP) nps = warp_sum(nps);
+            if (lane == 0) {
                 write_pose(p, c, g, e, vv, 0.0, nps, IFACE ? W.ibits : nullptr);
                 p.pose_counter[g] = 0;
             }
@@ -824,7 +896,7 @@ __host__ __device__ constexpr size_t wd_smem(int hcap) {
     return (size_t)hcap * sizeof(unsigned long long) + (size_t)(WD_THREADS / 32) * (sizeof(WSlots<G>) + sizeof(WDes<G>));
 }
 
-template <int G, bool IFACE>
+template <int G, bool IFACE, bool NP>
 __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(LaunchParams p) {
     constexpr int NW = WD_THREADS / 32;
     extern __shared__ __align__(16) unsigned char wd_smem_raw[];
@@ -832,7 +904,7 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
     __shared__ double s_red[4][32];
     __shared__ long long s_fix[32];
     __shared__ int s_spilled;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lane = w_lane(), wid = threadIdx.x >> 5;
     unsigned long long* const spill =
         p.spill ? reinterpret_cast<unsigned long long*>(p.spill + (size_t)blockIdx.x * p.spill_cap * SPILL_SLOT_BYTES)
                 : nullptr;
@@ -852,6 +924,8 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
         unsigned char* base = wd_smem_raw + (size_t)c.hcap * sizeof(unsigned long long);
         WSlots<G>& W = reinterpret_cast<WSlots<G>*>(base)[wid];
         WDes<G>* D = reinterpret_cast<WDes<G>*>(base + (size_t)NW * sizeof(WSlots<G>)) + wid;
+        w_descriptor(&W.c, &c, lane);
+        if (lane < 2) W.one[lane] = p.one;
         if (IFACE) W.ibuf[lane] = 0u;   // the slots move with the complex's hash size
         if (lane == 0) {
             W.rot = pose_matrix(p.poses + 7 * g);
@@ -860,8 +934,8 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
         }
         __syncthreads();   // hash cleared, poses set
         WAcc acc;
-        w_groups<G, true, IFACE>(c, W, D, &hash, p.status, wid, (c.nl + G - 1) / G, NW, acc, nullptr, nullptr,
-                                 p.far != nullptr);
+        w_groups<G, true, IFACE, NP>(W.c, W, D, &hash, p.status, lane, wid, (c.nl + G - 1) / G, NW, acc, nullptr,
+                                       p.far != nullptr);
         if (IFACE && W.ibits) w_iface_flush(W, c);   // before the block's barrier below
         __syncthreads();   // every pair has updated the hash
         // receptor side: fixed-point (2^-40) sum over hash slots; slot order
