@@ -96,6 +96,11 @@ struct LaunchParams {
     const int* item_pose0;       // [n_items] global pose offset
     const int* item_npose;       // [n_items]
     const long long* item_work0; // [n_items+1] cumulative work units
+    // warp kernel with split tiles: item_work0 counts units of `sub` groups,
+    // and item_group0 [n_items] is the item's first group partial; sub = 0:
+    // units are tiles
+    const long long* item_group0;
+    int sub;
     int n_items;
     long long total_work;
     int tile;                    // ligand atoms per work unit (non-desolv kernel)
@@ -106,7 +111,7 @@ struct LaunchParams {
     int raw_pairs;               // compat: scores holds (elec_raw, vdw) pairs
     int solv_only;               // compat cuda_cpydock_solv: scores[k] = S
     // scratch (self-resetting between launches)
-    double* partials;            // [total_work x 4] per-unit partial sums
+    double* partials;            // [x 4] partial sums per tile (or per group, split tiles)
     int* pose_counter;           // [N]
     unsigned long long* work_counter;  // [2]: next unit, CTAs done
     int* status;                 // [4]: error flags (capacity overflow, bad index)

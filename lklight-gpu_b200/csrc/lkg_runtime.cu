@@ -619,12 +619,48 @@ cudaError_t Scratch::ensure_spill(size_t bytes, cudaStream_t s) {
 }
 
 void Group::pack(char* dst) const {
-    const size_t ni = ic.size();
-    memcpy(dst, w0.data(), (ni + 1) * sizeof(long long));
-    int* t = (int*)(dst + (ni + 1) * sizeof(long long));
+    const size_t ni = ic.size(), nb = (ni + 1) * sizeof(long long);
+    memcpy(dst, w0.data(), nb);
+    if (sub) memcpy(dst + nb, ws.data(), nb);
+    if (sub) memcpy(dst + 2 * nb, g0.data(), nb);
+    int* t = (int*)(dst + 3 * nb);
     memcpy(t, ic.data(), ni * sizeof(int));
     memcpy(t + ni, ip0.data(), ni * sizeof(int));
     memcpy(t + 2 * ni, inp.data(), ni * sizeof(int));
+}
+
+// Units of the fast warp kernel: a tile of ligand atoms each, unless the
+// launch has fewer tiles than 2 for every warp slot of the GPU; then parts of
+// tiles, halved until there are as many, down to one group of atoms.  A warp
+// works through a unit's groups one after another, each a chain of dependent
+// loads of several us, so one pose took as long as a tile's 8-16 groups
+// (config-0 sizes: 194 us, now 63), and the warps that a small launch left
+// idle waited for the others (301 poses of a protein-density complex: 715 us,
+// now 308).  2, 8 and 1000 units a slot measured alike, but each group's
+// partial is 32 bytes to allocate (1 ms more on the first call with 1800 poses
+// at 8).  The score's bits are the same either way.
+constexpr int SPLIT_UNITS = 2;
+static void split_tiles(lkg_ctx* ctx, Group& G) {
+    if (G.ic.empty()) return;
+    const long long want = SPLIT_UNITS * (long long)ctx->sm_count * occupancy(ctx, false, false, ctx->tile, 0) *
+                           (128 / 32);
+    int sub = ctx->tile / ctx->group;
+    auto units = [&](int s) {
+        long long n = 0;
+        for (size_t i = 0; i < G.ic.size(); ++i) {
+            const long long ng = (ctx->cx[G.ic[i]]->d.nl + ctx->group - 1) / ctx->group;
+            n += G.inp[i] * ((ng + s - 1) / s);
+        }
+        return n;
+    };
+    while (sub > 1 && units(sub) < want) sub >>= 1;
+    if (sub == ctx->tile / ctx->group) return;
+    G.sub = sub;
+    for (size_t i = 0; i < G.ic.size(); ++i) {
+        const long long ng = (ctx->cx[G.ic[i]]->d.nl + ctx->group - 1) / ctx->group;
+        G.ws.push_back(G.ws.back() + G.inp[i] * ((ng + sub - 1) / sub));
+        G.g0.push_back(G.g0.back() + G.inp[i] * ng);
+    }
 }
 
 int build_groups(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, Group g[2], size_t* n_poses) {
@@ -657,11 +693,13 @@ int build_groups(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, G
         pose0 += counts[i];
     }
     *n_poses = (size_t)pose0;
+    split_tiles(ctx, g[0]);
     return set_ok();
 }
 
 long long group_blocks(lkg_ctx* ctx, const Group& G, bool exact) {
-    const long long work = std::max(1LL, G.w0.back());
+    const bool split = G.sub > 0 && !exact;
+    const long long work = std::max(1LL, split ? G.ws.back() : G.w0.back());
     long long blocks;
     if (G.kind == 0) blocks = (long long)ctx->sm_count * occupancy(ctx, false, exact, ctx->tile, 0);
     else blocks = (long long)ctx->sm_count * occupancy(ctx, true, exact, ctx->desolv_threads, G.hcap);
@@ -680,12 +718,15 @@ int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, cons
     const int ni = (int)G.ic.size();
     LaunchParams p{};
     p.cx = ctx->d_cx.as<ComplexDev>();
-    p.item_work0 = (const long long*)db;
-    p.item_complex = (const int*)(db + (size_t)(ni + 1) * sizeof(long long));
+    const bool split = G.kind == 0 && G.sub > 0 && !exact && !atom_e;
+    p.item_work0 = (const long long*)db + (split ? ni + 1 : 0);
+    p.item_group0 = (const long long*)db + 2 * (ni + 1);
+    p.sub = split ? G.sub : 0;
+    p.item_complex = (const int*)(db + 3 * (size_t)(ni + 1) * sizeof(long long));
     p.item_pose0 = p.item_complex + ni;
     p.item_npose = p.item_complex + 2 * ni;
     p.n_items = ni;
-    p.total_work = G.w0.back();
+    p.total_work = split ? G.ws.back() : G.w0.back();
     p.tile = ctx->tile;
     p.group = ctx->group;
     p.poses = d_poses;
@@ -759,7 +800,7 @@ int launch_items(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, c
     if ((st = build_groups(ctx, n_items, ids, counts, g, &n_poses))) return st;
     if (n_poses == 0) return set_ok();
     if ((st = sync_descriptors(ctx))) return st;
-    const size_t units = std::max<size_t>(g[0].w0.back(), 1);
+    const size_t units = std::max<size_t>(g[0].partials(), 1);
     LKG_CK(ctx->scratch.ensure(units, n_poses, ctx->stream, n_poses * (size_t)g[0].iface_words), "scratch");
     const size_t b0 = (g[0].bytes() + 255) & ~(size_t)255, b1 = (g[1].bytes() + 255) & ~(size_t)255;
     std::vector<char> packed(b0 + b1, 0);
@@ -1186,7 +1227,7 @@ int lkg_plan_create(lkg_ctx* ctx, int n_items, const int* ids, const int* counts
     cudaError_t e;
     if ((e = P->d_tables.reserve(b0 + b1)) != cudaSuccess ||
         (e = cudaMemcpy(P->d_tables.p, packed.data(), b0 + b1, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = P->scratch.ensure(std::max<size_t>(P->g[0].w0.back(), 1), std::max<size_t>(P->n_poses, 1), ctx->stream,
+        (e = P->scratch.ensure(std::max<size_t>(P->g[0].partials(), 1), std::max<size_t>(P->n_poses, 1), ctx->stream,
                                P->n_poses * (size_t)P->g[0].iface_words)) != cudaSuccess ||
         (e = P->scratch.ensure_spill(std::max(group_spill_bytes(ctx, P->g[1], false),
                                               group_spill_bytes(ctx, P->g[1], true)), ctx->stream)) != cudaSuccess ||

@@ -105,15 +105,21 @@ struct Scratch {
 };
 
 // one launch group's item tables: (complex, first pose, pose count) per item
-// and cumulative work units; `kind` 0 = tile kernels, 1 = fused desolvation
+// and cumulative work units; `kind` 0 = tile kernels, 1 = fused desolvation.
+// sub > 0: the fast warp kernel takes units of `sub` ligand groups instead of
+// tiles (ws: cumulative units, g0: cumulative group partials per item)
 struct Group {
     int kind = 0;
     std::vector<int> ic, ip0, inp;
     std::vector<long long> w0{0};
+    int sub = 0;
+    std::vector<long long> ws{0}, g0{0};
     int hcap = 64;
     int spill_cap = 0;     // desolvation spill slots per block: a power of two above the largest receptor
     int iface_words = 0;   // interface bit words per pose (the batch's largest)
-    size_t bytes() const { return (ic.size() + 1) * sizeof(long long) + ic.size() * 3 * sizeof(int); }
+    size_t bytes() const { return 3 * (ic.size() + 1) * sizeof(long long) + ic.size() * 3 * sizeof(int); }
+    // partial sums a launch writes (either precision)
+    size_t partials() const { return (size_t)std::max(w0.back(), sub ? g0.back() : 0LL); }
     void pack(char* dst) const;
 };
 

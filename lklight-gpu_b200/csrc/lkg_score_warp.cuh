@@ -81,6 +81,7 @@ struct WSlots {
     unsigned list[(G + 3) / 4][W_LIST + 16];   // receptor indices of each quad's candidates (and padding)
     int first[(G + 3) / 4], cnt[(G + 3) / 4];   // the part of each list that is scored
     float one[2];                     // 1, 1 (see w_d2)
+    double* part;                     // the unit's group partials (split tiles), or null
     int row[32];                      // per non-empty row of the current 32: first atom - the row's candidate offset
     ComplexDev c;                     // descriptor of the current unit's complex
     int ltag[G];                      // IFACE: restraint bit of the slot atom, -1 = none
@@ -468,12 +469,12 @@ __device__ __forceinline__ void w_dense(const ComplexDev& c, WSlots<G>& W, WDes<
 // rotation is in W.rot.  Plain and interface kernels: after each group its
 // sums, reduced over the warp, are added to acc.elec (lanes 0-15: the
 // electrostatics, lanes 16-31: the vdW), so acc is the sum of the groups'
-// sums in order.  DESOLV: acc holds the lane's own sums, and each slot atom's
+// sums in order; with W.part, each group's sums also go to its own 4 doubles
+// there.  DESOLV: acc holds the lane's own sums, and each slot atom's
 // g(min d^2) * des is added to acc.solv once its hits are all evaluated.
 template <int G, bool DESOLV, bool IFACE, bool NP, bool STAGE = false>
 __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes<G>* D, MinHash64* hash, int* status,
-                                         int lane, int g_first, int g_end, int g_step, WAcc& acc, WStage* S = nullptr,
-                                         bool far_sep = false) {
+                                         int lane, int g_first, int g_end, int g_step, WAcc& acc, WStage* S = nullptr, bool far_sep = false) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int NQ = (G + 3) / 4;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -778,6 +779,14 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) keep += __shfl_xor_sync(FULL, keep, o);
             acc.elec += keep;
+            if (W.part) {
+                double* gp = W.part + 4 * (size_t)(grp - g_first);
+                if ((lane & 15) == 0) gp[lane >> 4] = keep;
+                if (NP) {
+                    const int npg = (int)__reduce_add_sync(FULL, (unsigned)gsum.np);
+                    if (lane == 0) gp[3] = (double)npg;
+                }
+            }
         }
     }
     if (DESOLV) {
@@ -827,8 +836,13 @@ __global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchPara
         }
         const ComplexDev& c = W.c;
         const long long local = w - __ldg(p.item_work0 + b);
-        const int ntiles = c.ntiles;
-        const int pose = (int)(local / ntiles), tile = (int)(local % ntiles);
+        const int ngrp = (c.nl + G - 1) / G, gpt = p.tile / G;
+        // units of a pose, and this unit's groups: a tile's, or p.sub of them
+        const int gpu = p.sub ? p.sub : gpt;
+        const int nunits = (ngrp + gpu - 1) / gpu;
+        // (poses x units of one item fit 32 bits except in huge batches)
+        const int pose = local >> 32 ? (int)(local / nunits) : (int)((unsigned)local / (unsigned)nunits);
+        const int unit = (int)(local - (long long)pose * nunits);
         const long long g = (long long)__ldg(p.item_pose0 + b) + pose;
         if (p.pose_mask && !p.pose_mask[g]) continue;   // pose skipped: keeps its score
         __syncwarp();   // readers of the previous unit's pose are done
@@ -838,33 +852,51 @@ __global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchPara
             else if (c.iface_words) atomicOr(p.status, 2);   // a launch without room for the bits
         }
         __syncwarp();
-        const int gpt = p.tile / G;
-        const int g0 = tile * gpt, g1 = min(g0 + gpt, (c.nl + G - 1) / G);
+        const int g0 = unit * gpu, g1 = min(g0 + gpu, ngrp);
+        // partials: one per tile, or one per group when the tiles are split
+        // (a tile's sum is then made from its groups' in the same order, so
+        // the score's bits do not depend on the split)
+        const size_t first_part = p.sub ? __ldg(p.item_group0 + b) + (long long)pose * ngrp : w - unit;
+        if (lane == 0) W.part = p.sub ? p.partials + 4 * (first_part + g0) : nullptr;
+        __syncwarp();
         WAcc acc;
         w_groups<G, false, IFACE, NP, STAGE>(c, W, nullptr, nullptr, p.status, lane, g0, g1, 1, acc, S);
         if (IFACE && W.ibits) w_iface_flush(W, c);
-        // partial of work unit w; the pose's units are w - tile .. w - tile + ntiles - 1
-        double* part = p.partials + (size_t)w * 4;
-        if (lane == 0) part[0] = acc.elec;
-        if (lane == 16) part[1] = acc.elec;   // the vdW half
-        if (NP) {
-            const int npl = (int)__reduce_add_sync(FULL, (unsigned)acc.np);
-            if (lane == 0) part[3] = (double)npl;
+        double* const pose_part = p.partials + 4 * first_part;
+        if (!p.sub) {
+            double* const part = pose_part + 4 * (size_t)unit;
+            if ((lane & 15) == 0) part[lane >> 4] = acc.elec;   // electrostatics, vdW
+            if (NP) {
+                const int npl = (int)__reduce_add_sync(FULL, (unsigned)acc.np);
+                if (lane == 0) part[3] = (double)npl;
+            }
         }
-        __threadfence();   // partial (and interface bits) before the unit is published
+        __threadfence();   // partials (and interface bits) before the unit is published
         __syncwarp();
         int done = 0;
         if (lane == 0) done = atomicAdd(p.pose_counter + g, 1);
         done = __shfl_sync(FULL, done, 0);
-        if (done == ntiles - 1) {
+        if (done == nunits - 1) {
             __threadfence();
             // lane i sums tiles i, i + 32, ..., then a fixed tree
             double e = 0.0, vv = 0.0, nps = 0.0;
-            const double* pp = p.partials + (size_t)(w - tile) * 4;
-            for (int t = lane; t < ntiles; t += 32) {
-                e += __ldcg(pp + 4 * t);
-                vv += __ldcg(pp + 4 * t + 1);
-                if (NP) nps += __ldcg(pp + 4 * t + 3);
+            if (p.sub) {
+                for (int t = lane * gpt; t < ngrp; t += 32 * gpt) {
+                    double te = 0.0, tv = 0.0;
+                    for (int k = t; k < min(t + gpt, ngrp); ++k) {
+                        te += __ldcg(pose_part + 4 * k);
+                        tv += __ldcg(pose_part + 4 * k + 1);
+                        if (NP) nps += __ldcg(pose_part + 4 * k + 3);
+                    }
+                    e += te;
+                    vv += tv;
+                }
+            } else {
+                for (int t = lane; t < nunits; t += 32) {
+                    e += __ldcg(pose_part + 4 * t);
+                    vv += __ldcg(pose_part + 4 * t + 1);
+                    if (NP) nps += __ldcg(pose_part + 4 * t + 3);
+                }
             }
             e = warp_sum(e);
             vv = warp_sum(vv);

@@ -53,3 +53,20 @@ def test_lists_match_oracle(family, group, n):
     assert np.all(np.abs(got - ref) <= tol)
     assert np.array_equal(got, ctx.score(cid, poses))   # near pairs counted or not, the same bits
     ctx.close()
+
+
+@pytest.mark.parametrize("tile,group", [(64, 8), (128, 8), (128, 4), (256, 16), (256, 32)])
+@pytest.mark.parametrize("n", [3, 65, 300])
+def test_split_tiles_score_the_same_bits(tile, group, n):
+    # a launch of few poses is split into units of one to a few groups, a
+    # large one works in whole tiles: a pose's bits must not depend on it
+    rec, lig = _dense_receptor(), _ligand(n)
+    poses = random_poses(5, [0, 0, 0], 14.0, n)
+    ctx = lkg.Context(tile=tile, group=group)
+    cid = ctx.add_complex("dna", rec, lig)
+    alone = [ctx.score(cid, p, parts=True) for p in poses]
+    for count in (5, 300, 3000, 40000):
+        got, parts = ctx.score(cid, np.tile(poses, (count // 5, 1)), parts=True)
+        assert np.array_equal(got.reshape(-1, 5), np.tile([a[0][0] for a in alone], (count // 5, 1)))
+        assert np.array_equal(parts[:5], np.vstack([a[1] for a in alone]))
+    ctx.close()
