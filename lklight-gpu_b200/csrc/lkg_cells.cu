@@ -137,12 +137,14 @@ __global__ void k_pack(MolDev m, const int* __restrict__ order, int n, float4* _
     rorig[k] = i;
 }
 
-__global__ void k_interleave(const float4* __restrict__ pos, const float4* __restrict__ par, int n,
-                             float4* __restrict__ out) {
+__global__ void k_interleave(const float4* __restrict__ pos, const float4* __restrict__ par,
+                             const double2* __restrict__ solv, int n, float4* __restrict__ out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k > n) return;
     out[2 * (size_t)k] = k < n ? pos[k] : make_float4(3e30f, 3e30f, 3e30f, 0.f);
-    out[2 * (size_t)k + 1] = k < n ? par[k] : make_float4(0.f, 0.f, 0.f, 1.f);
+    float4 p = k < n ? par[k] : make_float4(0.f, 0.f, 0.f, 1.f);
+    if (p.w == 0.f && !solv_counts(solv[k])) p.w = 2.f;
+    out[2 * (size_t)k + 1] = p;
 }
 
 template <class T>
@@ -154,8 +156,9 @@ cudaError_t up(DBuf& b, const std::vector<T>& v, cudaStream_t s) {
 
 }  // namespace
 
-cudaError_t interleave_atoms(const float4* pos, const float4* par, int n, float4* out, cudaStream_t s) {
-    k_interleave<<<(unsigned)(n / 256 + 1), 256, 0, s>>>(pos, par, n, out);
+cudaError_t interleave_atoms(const float4* pos, const float4* par, const double2* solv, int n, float4* out,
+                             cudaStream_t s) {
+    k_interleave<<<(unsigned)(n / 256 + 1), 256, 0, s>>>(pos, par, solv, n, out);
     return cudaGetLastError();
 }
 

@@ -8,7 +8,8 @@
 //     rpos  float4 (x, y, z, q)              rpos64 double4 (same, f64)
 //     rpar  float4 (sqrt eps, r, heavy, excl) rpar64 double4 (sqrt eps, r, eps, heavy)
 //     rpk   both float4 of an atom side by side (32 bytes, one load), and
-//           one more atom far from everything
+//           one more atom far from everything; excl is 2 here for an atom
+//           that is not excluded but adds nothing to the desolvation sum
 //     rsolv float2 (des, asa)                rsolv64 double2
 //   ligand atoms ordered by recursive coordinate bisection of the reference
 //   frame into groups of `group` atoms (groups and tiles of consecutive
@@ -145,6 +146,12 @@ struct LaunchParams {
 // bytes per spill slot: the exact kernel's 8-byte value + 4-byte key (the
 // fast kernel's packed 8-byte slots use the first 8 x spill_cap bytes)
 constexpr int SPILL_SLOT_BYTES = 12;
+
+// whether an atom (des, asa) can add to the desolvation sum: g is 0 without a
+// reference area, and des scales it (a non-finite des keeps its product)
+__host__ __device__ inline bool solv_counts(double2 s) {
+    return s.x != 0.0 && (s.y > 0.0 || !(s.x - s.x == 0.0));
+}
 
 constexpr double FACTOR = 332.0;
 constexpr double EPSILON = 4.0;

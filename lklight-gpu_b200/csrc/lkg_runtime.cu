@@ -183,7 +183,8 @@ namespace {
 // out of reach of everything that adds nothing (it pads the candidate lists)
 int interleave_receptor(lkg_ctx* ctx, ComplexRec& cr, int n) {
     LKG_CK(cr.rpk.reserve(((size_t)n + 1) * 2 * sizeof(float4)), "receptor arrays");
-    LKG_CK(interleave_atoms(cr.rpos.as<float4>(), cr.rpar.as<float4>(), n, cr.rpk.as<float4>(), ctx->stream),
+    LKG_CK(interleave_atoms(cr.rpos.as<float4>(), cr.rpar.as<float4>(), cr.rsolv64.as<double2>(), n,
+                            cr.rpk.as<float4>(), ctx->stream),
            "receptor arrays");
     ctx->launches++;
     LKG_CK(cudaStreamSynchronize(ctx->stream), "receptor arrays");

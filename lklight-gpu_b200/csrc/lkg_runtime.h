@@ -170,7 +170,8 @@ int build_receptor_device(lkg_ctx* ctx, const MolIn& R, ComplexRec& cr, const fl
                           const float inv_e[3]);
 // both float4 of n atoms side by side, then an atom out of reach of everything
 // that adds nothing (ComplexDev::rpk; out: 2 (n + 1) float4)
-cudaError_t interleave_atoms(const float4* pos, const float4* par, int n, float4* out, cudaStream_t s);
+cudaError_t interleave_atoms(const float4* pos, const float4* par, const double2* solv, int n, float4* out,
+                             cudaStream_t s);
 // replace the ligand of an existing complex (cuda_full_score)
 int complex_set_ligand(lkg_ctx* ctx, int id, const MolIn& lig);
 // a complex changed: descriptors to upload, captured graphs out of date

@@ -51,8 +51,9 @@ constexpr int WK_BLOCKS = 7;
 // per-warp desolvation state of the two slot sets (cpydock): the slot
 // atoms' f64 positions, their running minimum d^2 to non-excluded receptor
 // atoms (f64 bits; non-negative doubles order like their bit patterns), and
-// the hits within 6.4 A that wait for it (slot << 26 | receptor index): fewer
-// than 32 wait when a step of 64 tests adds its own
+// the hits within 6.4 A that wait for it (slot << 26 | receptor index, bit 31
+// when the receptor atom's minimum is wanted too): fewer than 32 wait when a
+// step of 64 tests adds its own
 template <int G>
 struct WDes {
     double lx[2 * G], ly[2 * G], lz[2 * G];
@@ -83,7 +84,6 @@ struct WSlots {
     float one[2];                     // 1, 1 (see w_d2)
     double* part;                     // the unit's group partials (split tiles), or null
     int row[32];                      // per non-empty row of the current 32: first atom - the row's candidate offset
-    ComplexDev c;                     // descriptor of the current unit's complex
     int ltag[G];                      // IFACE: restraint bit of the slot atom, -1 = none
     float lf[G];                      // DESOLV: largest f32 d^2 of interest (-1: atom excluded)
     unsigned* ibits;                  // IFACE: interface bits of the current pose in HBM (null: none)
@@ -127,14 +127,20 @@ __device__ __forceinline__ bool w_bar_wait(uint32_t bar, uint32_t parity) {
 // shared table holds (a ligand sunk into a large receptor) continues in the
 // block's own table in global memory, of more slots than the complex has
 // receptor atoms, so an insert there always finds its key or an empty slot.
-// A key enters the global table only after the shared table was found full
-// without it, and a full shared table stays full, so the two tables hold
-// disjoint keys and the receptor sum runs over both.  The block empties the
+// A key enters the global table only after its PROBES slots of the shared
+// table were found taken by others, and taken slots stay taken, so the two
+// tables hold disjoint keys and the receptor sum runs over both.  The block empties the
 // global slots it used when it sums them.
 struct MinHash64 {
     static constexpr unsigned long long EMPTY = ~0ull;
     static constexpr unsigned long long KEY_MASK = (1ull << 27) - 1;
     static constexpr double SCALE = (double)((1ull << 37) - 1) / SOLV2_D;
+    // slots of the shared table a key may take.  Without a limit a pose that
+    // filled the table probed all of it (2048 slots) for each key that it then
+    // spilled: 1500 poses with a 12,000-atom ligand sunk into a 101,000-atom
+    // receptor took 49.6 ms, now 5.9 (16 slots: 6.6, and 8 % more than 64
+    // where the table is three quarters full; 32: 6.3)
+    static constexpr int PROBES = 64;
     unsigned long long* slot;
     int cap;
     unsigned long long* spill;   // the block's global table (all EMPTY between poses), or null
@@ -149,13 +155,15 @@ struct MinHash64 {
         for (int s = threadIdx.x; s < cap; s += blockDim.x) slot[s] = EMPTY;
         if (threadIdx.x == 0) *spilled = 0;
     }
-    // linear probing over tab[0..n) (n a power of two); false when full.
+    // linear probing over tab[0..n) (n a power of two); false when full (the
+    // shared table: when the key's PROBES slots are).
     // GLOBAL: the table is in global memory, where the atomics act in L2:
     // plain reads there bypass L1 (__ldcg), which could hold a stale line
     template <bool GLOBAL>
     __device__ static bool put(unsigned long long* tab, int n, int k, unsigned long long w) {
         unsigned h = ((unsigned)k * 2654435761u) & (unsigned)(n - 1);
-        for (int probe = 0; probe < n; ++probe) {
+        const int most = GLOBAL ? n : (n < PROBES ? n : PROBES);
+        for (int probe = 0; probe < most; ++probe) {
             unsigned long long v = GLOBAL ? __ldcg(tab + h) : tab[h];
             if (v == EMPTY) {
                 v = atomicCAS(tab + h, EMPTY, w);
@@ -258,13 +266,13 @@ __device__ __forceinline__ int w_lane() {
     return (int)l;
 }
 
-// the descriptor of a unit's complex into the warp's shared memory (its
+// the descriptor of a unit's complex into shared memory by n threads (its
 // fields are read all through a unit; from global memory each read waited)
-__device__ __forceinline__ void w_descriptor(ComplexDev* dst, const ComplexDev* src, int lane) {
+__device__ __forceinline__ void w_descriptor(ComplexDev* dst, const ComplexDev* src, int lane, int n) {
     static_assert(sizeof(ComplexDev) % 8 == 0, "copied in 8-byte words");
     const unsigned long long* s = reinterpret_cast<const unsigned long long*>(src);
     unsigned long long* d = reinterpret_cast<unsigned long long*>(dst);
-    for (int i = lane; i < (int)(sizeof(ComplexDev) / 8); i += 32) d[i] = __ldg(s + i);
+    for (int i = lane; i < (int)(sizeof(ComplexDev) / 8); i += n) d[i] = __ldg(s + i);
 }
 
 constexpr unsigned long long W_NOMIN = 0x7fefffffffffffffull;   // largest finite double
@@ -295,12 +303,12 @@ __device__ __forceinline__ void w_minima(const ComplexDev& c, WDes<G>* D, MinHas
     const int lane = threadIdx.x & 31;
     if (lane >= n) return;
     const unsigned e = D->hit[first + lane];
-    const int l = (int)(e >> 26), k = (int)(e & 0x3ffffffu);
+    const int l = (int)(e >> 26 & 31u), k = (int)(e & 0x3ffffffu);
     const double4 a = c.rpos64[k];
     const double ex = D->lx[l] - a.x, ey = D->ly[l] - a.y, ez = D->lz[l] - a.z;
     const double d2 = ex * ex + ey * ey + ez * ez;
     atomicMin(&D->lmin[l], (unsigned long long)__double_as_longlong(d2));
-    if (d2 <= SOLV2_D && !hash->insert(k, d2)) atomicOr(status, 1);
+    if ((e >> 31) && d2 <= SOLV2_D && !hash->insert(k, d2)) atomicOr(status, 1);
 }
 
 // d^2 of a receptor atom and both slots of a pair, from the compensated
@@ -365,7 +373,11 @@ __device__ __forceinline__ void w_dense(const ComplexDev& c, WSlots<G>& W, WDes<
     // IFACE: a slot of the pair is tagged (untagged receptor atoms matter then)
     const bool tagged = IFACE && iset && (W.ltag[slot0] >= 0 || W.ltag[slot0 + 1] >= 0);
     float lf0 = 0.f, lf1 = 0.f;
-    if (DESOLV) { lf0 = W.lf[slot0]; lf1 = W.lf[slot0 + 1]; }
+    bool need0 = false, need1 = false;   // DESOLV: the slot's own minimum is wanted
+    if (DESOLV) {
+        lf0 = W.lf[slot0]; lf1 = W.lf[slot0 + 1];
+        need0 = lf0 > SOLV2_F * 1.0005f; need1 = lf1 > SOLV2_F * 1.0005f;
+    }
     auto step = [&](const WAtom& A, unsigned k) {
         const F2 d2 = w_d2<DESOLV || IFACE>(P, A, one);
         float d20, d21, t0, t1;
@@ -430,13 +442,15 @@ __device__ __forceinline__ void w_dense(const ComplexDev& c, WSlots<G>& W, WDes<
             }
         }
         if (DESOLV) {
-            const bool s0 = d20 <= lf0 && A.p.w == 0.f, s1 = d21 <= lf1 && A.p.w == 0.f;
+            const bool want = A.p.w == 0.f, may = A.p.w != 1.f;
+            const bool s0 = d20 <= lf0 && may && (want || need0), s1 = d21 <= lf1 && may && (want || need1);
             const unsigned b0 = __ballot_sync(FULL, s0), b1 = __ballot_sync(FULL, s1);
             if (b0 | b1) {
                 const unsigned lt_mask = (1u << lane) - 1u;
                 const int n0 = __popc(b0);
-                if (s0) D->hit[nhit + __popc(b0 & lt_mask)] = ((unsigned)(set + slot0) << 26) | k;
-                if (s1) D->hit[nhit + n0 + __popc(b1 & lt_mask)] = ((unsigned)(set + slot0 + 1) << 26) | k;
+                const unsigned e = ((unsigned)(set + slot0) << 26) | k | (want ? 0x80000000u : 0u);
+                if (s0) D->hit[nhit + __popc(b0 & lt_mask)] = e;
+                if (s1) D->hit[nhit + n0 + __popc(b1 & lt_mask)] = e + (1u << 26);
                 nhit += n0 + __popc(b1);
                 __syncwarp();
                 int head = 0;
@@ -465,16 +479,17 @@ __device__ __forceinline__ void w_dense(const ComplexDev& c, WSlots<G>& W, WDes<
     }
 }
 
-// Scores groups g_first, g_first + g_step, ... (< g_end) of one pose whose
-// rotation is in W.rot.  Plain and interface kernels: after each group its
+// Scores groups group_of(first), group_of(first + step), ... (indices < end) of
+// one pose whose rotation is in W.rot.  Plain and interface kernels: after each group its
 // sums, reduced over the warp, are added to acc.elec (lanes 0-15: the
 // electrostatics, lanes 16-31: the vdW), so acc is the sum of the groups'
 // sums in order; with W.part, each group's sums also go to its own 4 doubles
 // there.  DESOLV: acc holds the lane's own sums, and each slot atom's
 // g(min d^2) * des is added to acc.solv once its hits are all evaluated.
-template <int G, bool DESOLV, bool IFACE, bool NP, bool STAGE = false>
+template <int G, bool DESOLV, bool IFACE, bool NP, bool STAGE = false, class GroupOf>
 __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes<G>* D, MinHash64* hash, int* status,
-                                         int lane, int g_first, int g_end, int g_step, WAcc& acc, WStage* S = nullptr, bool far_sep = false) {
+                                         int lane, int first, int end, int step, GroupOf group_of, WAcc& acc,
+                                         WStage* S = nullptr, bool far_sep = false) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int NQ = (G + 3) / 4;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -499,7 +514,8 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
         if (set) jdes1 = -1; else jdes0 = -1;
     };
     int it = 0;
-    for (int grp = g_first; grp < g_end; grp += g_step, ++it) {
+    for (int gk = first; gk < end; gk += step, ++it) {
+        const int grp = group_of(gk);
         const int set = DESOLV ? (it & 1) * G : 0;
         __syncwarp();
         if (DESOLV) {
@@ -551,7 +567,10 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
                 if (DESOLV) {
                     D->lx[set + lane] = xd; D->ly[set + lane] = yd; D->lz[set + lane] = zd;
                     D->lmin[set + lane] = W_NOMIN;
-                    W.lf[lane] = lp4.w != 0.f ? -1.f : SOLV2_F * 1.001f;
+                    // (two thresholds, both above 6.4^2: the larger one marks an
+                    // atom whose own minimum is wanted)
+                    const bool need = atom && solv_counts(c.lsolv64[j]);
+                    W.lf[lane] = lp4.w != 0.f ? -1.f : (need ? SOLV2_F * 1.001f : SOLV2_F * 1.0004f);
                     if (set) jdes1 = atom ? j : -1; else jdes0 = atom ? j : -1;
                 }
                 // far field with the reference's f64 interpolation (a per-atom
@@ -582,15 +601,6 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
         }
         // 2. receptor rows within reach of the group sphere
         const float R2 = R * R;
-        // cpydock kernel: no receptor atom within R of the centre, so the
-        // group has no candidate and its rows are not enumerated (most groups
-        // of a large ligand at the interface: with a 12,000-atom ligand on a
-        // 101,000-atom receptor the step is 4.5 % faster; the plain kernel,
-        // whose ligands are smaller, measured 1 % slower with the test)
-        if (DESOLV && c.rlb && R < c.rlb_m && w_receptor_bound(c, gx, gy, gz) > R) {
-            acc.elec += gsum.elec;
-            continue;
-        }
         const int cz0 = max(0, (int)floorf((gz - R - c.oz) * c.inv_h));
         const int cz1 = min(c.ncz - 1, (int)floorf((gz + R - c.oz) * c.inv_h));
         const int cy0 = max(0, (int)floorf((gy - R - c.oy) * c.inv_h));
@@ -780,7 +790,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
             for (int o = 8; o > 0; o >>= 1) keep += __shfl_xor_sync(FULL, keep, o);
             acc.elec += keep;
             if (W.part) {
-                double* gp = W.part + 4 * (size_t)(grp - g_first);
+                double* gp = W.part + 4 * (size_t)(gk - first);
                 if ((lane & 15) == 0) gp[lane >> 4] = keep;
                 if (NP) {
                     const int npg = (int)__reduce_add_sync(FULL, (unsigned)gsum.np);
@@ -807,7 +817,10 @@ __global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchPara
     extern __shared__ __align__(16) unsigned char wk_smem[];
     const int lane = w_lane();
     WSlots<G>& W = reinterpret_cast<WSlots<G>*>(wk_smem)[threadIdx.x >> 5];
-    WStage* S = STAGE ? reinterpret_cast<WStage*>(wk_smem + (WK_THREADS / 32) * sizeof(WSlots<G>)) + (threadIdx.x >> 5)
+    // descriptor of the current unit's complex
+    ComplexDev& c = reinterpret_cast<ComplexDev*>(wk_smem + (WK_THREADS / 32) * sizeof(WSlots<G>))[threadIdx.x >> 5];
+    WStage* S = STAGE ? reinterpret_cast<WStage*>(wk_smem + (WK_THREADS / 32) * (sizeof(WSlots<G>) + sizeof(ComplexDev))) +
+                            (threadIdx.x >> 5)
                       : nullptr;
     if (STAGE) {
         if (lane == 0) {
@@ -820,7 +833,7 @@ __global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchPara
     if (IFACE) W.ibuf[lane] = 0u;
     if (lane < 2) W.one[lane] = p.one;
     __syncwarp();
-    int cur = -1;   // complex whose descriptor W.c holds
+    int cur = -1;   // complex whose descriptor c holds
     for (;;) {
         unsigned long long wq = 0;
         if (lane == 0) wq = atomicAdd(p.work_counter, 1ull);
@@ -830,11 +843,10 @@ __global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchPara
         const int cid = __ldg(p.item_complex + b);
         if (cid != cur) {
             __syncwarp();
-            w_descriptor(&W.c, p.cx + cid, lane);
+            w_descriptor(&c, p.cx + cid, lane, 32);
             cur = cid;
             __syncwarp();
         }
-        const ComplexDev& c = W.c;
         const long long local = w - __ldg(p.item_work0 + b);
         const int ngrp = (c.nl + G - 1) / G, gpt = p.tile / G;
         // units of a pose, and this unit's groups: a tile's, or p.sub of them
@@ -860,7 +872,7 @@ __global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchPara
         if (lane == 0) W.part = p.sub ? p.partials + 4 * (first_part + g0) : nullptr;
         __syncwarp();
         WAcc acc;
-        w_groups<G, false, IFACE, NP, STAGE>(c, W, nullptr, nullptr, p.status, lane, g0, g1, 1, acc, S);
+        w_groups<G, false, IFACE, NP, STAGE>(c, W, nullptr, nullptr, p.status, lane, g0, g1, 1, [](int k) { return k; }, acc, S);
         if (IFACE && W.ibits) w_iface_flush(W, c);
         double* const pose_part = p.partials + 4 * first_part;
         if (!p.sub) {
@@ -912,8 +924,9 @@ __global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchPara
 }
 
 // cpydock: one block per pose (the receptor-side minima live in the block's
-// shared-memory hash); warp k takes the pose's groups k, k + NW, ... (a fixed
-// assignment: the sums do not depend on scheduling).  Block layout of the
+// shared-memory hash); the pose's groups within the receptor's reach are listed
+// first (a lane a group), and warp k takes the near groups k, k + NW, ... (a
+// fixed assignment: the sums do not depend on scheduling).  Block layout of the
 // dynamic shared memory: hash (hcap x 8 B), then NW x WSlots, NW x WDes.
 // 8 warps a block, three blocks an SM (24 warps resident, 80 registers):
 // the block's warps wait for one another at the end of every pose, and
@@ -922,6 +935,21 @@ __global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchPara
 // at 5 blocks: 34.2 ms).
 constexpr int WD_THREADS = 256;
 constexpr int WD_BLOCKS = 3;
+// groups whose reach is tested at a time (most groups of a large ligand at the
+// interface are too far from the receptor: in a CPU model of a 12,000-atom
+// ligand on a 101,000-atom receptor 84-89 % of the groups of 16)
+constexpr int WD_NEAR = 1024;
+
+// whether a receptor atom can lie within reach of group gi (its sphere grown by
+// SCAN_R), by the receptor's distance bound at the posed centre
+__device__ __forceinline__ bool w_near(const ComplexDev& c, const Rot& rot, int gi) {
+    const float4 gs = __ldg(c.lgrp + gi);
+    const float R = SCAN_R + gs.w;
+    if (!c.rlb || !(R < c.rlb_m)) return true;
+    double x, y, z;
+    apply(rot, (double)gs.x, (double)gs.y, (double)gs.z, x, y, z);
+    return !(w_receptor_bound(c, (float)x, (float)y, (float)z) > R);
+}
 
 template <int G>
 __host__ __device__ constexpr size_t wd_smem(int hcap) {
@@ -936,6 +964,9 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
     __shared__ double s_red[4][32];
     __shared__ long long s_fix[32];
     __shared__ int s_spilled;
+    __shared__ ComplexDev s_c;
+    __shared__ unsigned s_near[WD_NEAR / 32];
+    __shared__ unsigned short s_list[WD_NEAR];
     const int lane = w_lane(), wid = threadIdx.x >> 5;
     unsigned long long* const spill =
         p.spill ? reinterpret_cast<unsigned long long*>(p.spill + (size_t)blockIdx.x * p.spill_cap * SPILL_SLOT_BYTES)
@@ -947,16 +978,18 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
         __syncthreads();
         if (w >= p.total_work) break;
         const int b = find_item(p.item_work0, p.n_items, w);
-        const ComplexDev& c = p.cx[__ldg(p.item_complex + b)];
+        const ComplexDev* cg = p.cx + __ldg(p.item_complex + b);
         const int pose = (int)(w - __ldg(p.item_work0 + b));
         const long long g = (long long)__ldg(p.item_pose0 + b) + pose;
         if (p.pose_mask && !p.pose_mask[g]) continue;   // block-uniform: pose skipped
+        if (threadIdx.x < 32) w_descriptor(&s_c, cg, lane, 32);
+        __syncthreads();
+        const ComplexDev& c = s_c;
         MinHash64 hash;
         hash.init(reinterpret_cast<char*>(wd_smem_raw), c.hcap, spill, p.spill_cap, &s_spilled);
         unsigned char* base = wd_smem_raw + (size_t)c.hcap * sizeof(unsigned long long);
         WSlots<G>& W = reinterpret_cast<WSlots<G>*>(base)[wid];
         WDes<G>* D = reinterpret_cast<WDes<G>*>(base + (size_t)NW * sizeof(WSlots<G>)) + wid;
-        w_descriptor(&W.c, &c, lane);
         if (lane < 2) W.one[lane] = p.one;
         if (IFACE) W.ibuf[lane] = 0u;   // the slots move with the complex's hash size
         if (lane == 0) {
@@ -966,8 +999,40 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
         }
         __syncthreads();   // hash cleared, poses set
         WAcc acc;
-        w_groups<G, true, IFACE, NP>(W.c, W, D, &hash, p.status, lane, wid, (c.nl + G - 1) / G, NW, acc, nullptr,
-                                       p.far != nullptr);
+        const bool far_sep = p.far != nullptr;
+        const int ngrp = (c.nl + G - 1) / G;
+        for (int g0 = 0; g0 < ngrp; g0 += WD_NEAR) {
+            // which of up to WD_NEAR groups a receptor atom can reach, a lane
+            // a group (an inline far field wants them all)
+            const int words = min(WD_NEAR, ngrp - g0 + 31) / 32;
+            for (int i = wid; i < words; i += NW) {
+                const int gi = g0 + i * 32 + lane;
+                const bool near = gi < ngrp && (((c.flags & F_FAR) && !far_sep) || w_near(c, W.rot, gi));
+                const unsigned m = __ballot_sync(0xffffffffu, near);
+                if (lane == 0) s_near[i] = m;
+            }
+            __syncthreads();
+            // the near groups in order: lane i counts word i's, each warp
+            // writes its words' out
+            const unsigned mine = lane < words ? s_near[lane] : 0u;
+            int inc = __popc(mine);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += v;
+            }
+            const int total = __shfl_sync(0xffffffffu, inc, 31);
+            for (int i = wid; i < words; i += NW) {
+                const unsigned m = __shfl_sync(0xffffffffu, mine, i);
+                const int before = __shfl_sync(0xffffffffu, inc, i) - __popc(m);
+                if (m >> lane & 1u) s_list[before + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(i * 32 + lane);
+            }
+            __syncthreads();
+            // warp k scores the near groups k, k + NW, ...
+            w_groups<G, true, IFACE, NP>(c, W, D, &hash, p.status, lane, wid, total, NW,
+                                         [&](int k) { return g0 + s_list[k]; }, acc, nullptr, far_sep);
+            if (g0 + WD_NEAR < ngrp) __syncthreads();   // the list is read
+        }
         if (IFACE && W.ibits) w_iface_flush(W, c);   // before the block's barrier below
         __syncthreads();   // every pair has updated the hash
         // receptor side: fixed-point (2^-40) sum over hash slots; slot order
