@@ -168,7 +168,7 @@ constexpr double MEMBRANE_PENALTY = 999.0;   // MEMBRANE_PENALTY_SCORE (constant
 // launches (defined in lkg_kernels_*.cu)
 cudaError_t launch_score_fast(const LaunchParams& p, int threads, int blocks, cudaStream_t s);
 cudaError_t launch_desolv_fast(const LaunchParams& p, int threads, int blocks, int hcap, cudaStream_t s);
-cudaError_t launch_score_exact(const LaunchParams& p, int threads, int blocks, cudaStream_t s);
+cudaError_t launch_score_exact(const LaunchParams& p, int blocks, cudaStream_t s);
 cudaError_t launch_desolv_exact(const LaunchParams& p, int threads, int blocks, int hcap, cudaStream_t s);
 // the far-field pass of a fast cpydock launch group (fills p.far)
 cudaError_t launch_far_poses(const LaunchParams& p, int blocks, cudaStream_t s);

@@ -15,7 +15,7 @@ namespace lkg {
 
 int max_blocks_score_fast(int threads, int group);
 int max_blocks_desolv_fast(int threads, int hcap, int group);
-int max_blocks_score_exact(int threads);
+int max_blocks_score_exact(int group);
 int max_blocks_desolv_exact(int threads, int hcap);
 
 namespace {
@@ -447,7 +447,7 @@ int occupancy(lkg_ctx* ctx, bool desolv, bool exact, int threads, int hcap) {
     if (o.threads == threads && o.hcap == hcap && o.blocks > 0) return o.blocks;
     int b;
     if (desolv) b = exact ? max_blocks_desolv_exact(threads, hcap) : max_blocks_desolv_fast(threads, hcap, ctx->group);
-    else b = exact ? max_blocks_score_exact(threads) : max_blocks_score_fast(threads, ctx->group);
+    else b = exact ? max_blocks_score_exact(ctx->group) : max_blocks_score_fast(threads, ctx->group);
     o.threads = threads; o.hcap = hcap; o.blocks = std::max(1, b);
     return o.blocks;
 }
@@ -699,7 +699,7 @@ int build_groups(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, G
 }
 
 long long group_blocks(lkg_ctx* ctx, const Group& G, bool exact) {
-    const bool split = G.sub > 0 && !exact;
+    const bool split = G.sub > 0;
     const long long work = std::max(1LL, split ? G.ws.back() : G.w0.back());
     long long blocks;
     if (G.kind == 0) blocks = (long long)ctx->sm_count * occupancy(ctx, false, exact, ctx->tile, 0);
@@ -719,7 +719,7 @@ int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, cons
     const int ni = (int)G.ic.size();
     LaunchParams p{};
     p.cx = ctx->d_cx.as<ComplexDev>();
-    const bool split = G.kind == 0 && G.sub > 0 && !exact && !atom_e;
+    const bool split = G.kind == 0 && G.sub > 0 && !atom_e;
     p.item_work0 = (const long long*)db + (split ? ni + 1 : 0);
     p.item_group0 = (const long long*)db + 2 * (ni + 1);
     p.sub = split ? G.sub : 0;
@@ -757,7 +757,7 @@ int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, cons
     cudaError_t e;
     const long long blocks = group_blocks(ctx, G, exact);
     if (G.kind == 0) {
-        e = exact ? launch_score_exact(p, ctx->tile, (int)blocks, ctx->stream)
+        e = exact ? launch_score_exact(p, (int)blocks, ctx->stream)
                   : launch_score_fast(p, ctx->tile, (int)blocks, ctx->stream);
     } else {
         int threads = ctx->desolv_threads;

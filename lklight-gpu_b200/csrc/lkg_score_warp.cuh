@@ -47,6 +47,10 @@ constexpr int W_LIST = 128;
 // few spills in the cold parts).  Sixteen complexes of 2,000 poses: 12.5 ms at
 // 5 blocks, 12.4 at 6, 12.1 at 7, 12.5 at 8.
 constexpr int WK_BLOCKS = 7;
+// f64 mode: bound by the latency of its f64 chains, so more warps win over
+// fewer spills (200 poses: 440 us at 4 blocks, 399 at 5, 387 at 6, 370 at 7,
+// 360 at 8)
+constexpr int WK_BLOCKS_EXACT = 8;
 
 // per-warp desolvation state of the two slot sets (cpydock): the slot
 // atoms' f64 positions, their running minimum d^2 to non-excluded receptor
@@ -288,6 +292,12 @@ __device__ __forceinline__ float w_receptor_bound(const ComplexDev& c, float x, 
 }
 
 
+// The f64 mode's slots: a group's ligand atoms as the reference holds them.
+template <int G>
+struct WExact {
+    double x[G], y[G], z[G], q[G], sv[G], r[G], eps[G], h[G];
+};
+
 // The warp's sums over its groups (cpydock: per lane; else per group, reduced).
 struct WAcc {
     double elec = 0.0, vdw = 0.0, solv = 0.0;
@@ -479,6 +489,36 @@ __device__ __forceinline__ void w_dense(const ComplexDev& c, WSlots<G>& W, WDes<
     }
 }
 
+// The f64 mode of w_dense: the listed candidates in the reference's arithmetic
+// (compiled without contraction), 16 a step, lane = (candidate, two slots).
+// The lists only have to hold every pair within the cutoff; each pair is in or
+// out by its own f64 d^2.
+template <int G, bool IFACE, bool NP>
+__device__ __forceinline__ void w_dense_exact(const ComplexDev& c, const WSlots<G>& W, const WExact<G>& X,
+                                              unsigned* iset, int lane, int quad, int first, int n, WAcc& acc) {
+    const int slot0 = quad * 4 + (lane & 1) * 2;
+    for (int i = lane >> 1; i < n; i += 16) {
+        const int k = (int)W.list[quad][first + i];
+        const double4 a = c.rpos64[k];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int l = slot0 + h;
+            const double dx = X.x[l] - a.x, dy = X.y[l] - a.y, dz = X.z[l] - a.z;
+            const double d2 = dx * dx + dy * dy + dz * dz;
+            if (!(d2 <= 100.0)) continue;
+            if (NP) ++acc.np;
+            pair_exact(c.flags, c.lj_form, X.q[l], X.sv[l], X.r[l], X.eps[l], X.h[l] != 0.0, a, c.rpar64[k], d2,
+                       acc.elec, acc.vdw);
+            if (IFACE && iset && d2 <= IFACE2_D) {
+                const int2 rt = __ldg(c.rtag + k);
+                iface_set(iset, rt.x);
+                iface_set(iset, rt.y);
+                iface_set(iset, W.ltag[l]);
+            }
+        }
+    }
+}
+
 // Scores groups group_of(first), group_of(first + step), ... (indices < end) of
 // one pose whose rotation is in W.rot.  Plain and interface kernels: after each group its
 // sums, reduced over the warp, are added to acc.elec (lanes 0-15: the
@@ -486,10 +526,10 @@ __device__ __forceinline__ void w_dense(const ComplexDev& c, WSlots<G>& W, WDes<
 // sums in order; with W.part, each group's sums also go to its own 4 doubles
 // there.  DESOLV: acc holds the lane's own sums, and each slot atom's
 // g(min d^2) * des is added to acc.solv once its hits are all evaluated.
-template <int G, bool DESOLV, bool IFACE, bool NP, bool STAGE = false, class GroupOf>
+template <int G, bool DESOLV, bool IFACE, bool NP, bool STAGE, bool EXACT, class GroupOf>
 __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes<G>* D, MinHash64* hash, int* status,
                                          int lane, int first, int end, int step, GroupOf group_of, WAcc& acc,
-                                         WStage* S = nullptr, bool far_sep = false) {
+                                         WStage* S = nullptr, WExact<G>* X = nullptr, bool far_sep = false) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int NQ = (G + 3) / 4;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -551,8 +591,15 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
             apply(W.rot, b.x, b.y, b.z, xd, yd, zd);
             float x = (float)xd, y = (float)yd, z = (float)zd;
             if (lane < G) {
-                const float4 lp4 = atom ? __ldg(c.lpar + j) : make_float4(0.f, 0.f, 0.f, 0.f);
                 const float q = (float)b.w;
+                if constexpr (EXACT) {
+                    const double4 lp = atom ? c.lpar64[j] : make_double4(0.0, 0.0, 0.0, 0.0);
+                    X->x[lane] = atom ? xd : 1e30;   // never within reach of a receptor atom
+                    X->y[lane] = atom ? yd : 1e30;
+                    X->z[lane] = atom ? zd : 1e30;
+                    X->q[lane] = b.w; X->sv[lane] = lp.x; X->r[lane] = lp.y; X->eps[lane] = lp.z; X->h[lane] = lp.w;
+                } else {
+                const float4 lp4 = atom ? __ldg(c.lpar + j) : make_float4(0.f, 0.f, 0.f, 0.f);
                 WPair& P = W.pair[lane >> 1];
                 const int h = lane & 1;
                 P.rx[h] = (float)(xd - (double)x);
@@ -563,7 +610,6 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
                 P.z[h] = atom ? z : 1e30f;
                 P.q[h] = q; P.sv[h] = lp4.x; P.r[h] = lp4.y;
                 P.h[h] = lp4.z != 0.f ? 0.75f : 0.f;
-                if (IFACE) W.ltag[lane] = (atom && c.ltag) ? __ldg(c.ltag + j) : -1;
                 if (DESOLV) {
                     D->lx[set + lane] = xd; D->ly[set + lane] = yd; D->lz[set + lane] = zd;
                     D->lmin[set + lane] = W_NOMIN;
@@ -573,11 +619,13 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
                     W.lf[lane] = lp4.w != 0.f ? -1.f : (need ? SOLV2_F * 1.001f : SOLV2_F * 1.0004f);
                     if (set) jdes1 = atom ? j : -1; else jdes0 = atom ? j : -1;
                 }
+                }
+                if (IFACE) W.ltag[lane] = (atom && c.ltag) ? __ldg(c.ltag + j) : -1;
                 // far field with the reference's f64 interpolation (a per-atom
                 // cost; f32 here would add up over thousands of charged atoms)
                 // (the cpydock kernel takes it from k_far_poses instead when
                 // that pass ran: far_sep)
-                if (atom && (flags & F_FAR) && !(DESOLV && far_sep) && q != 0.f)
+                if (atom && (flags & F_FAR) && !(DESOLV && far_sep) && (EXACT ? b.w != 0.0 : q != 0.f))
                     gsum.elec = b.w * sample_phi(c, xd, yd, zd);
             }
             if (G == 32) {
@@ -746,11 +794,16 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
             for (int s = 0; s < NQ; ++s) {
                 // the length to score, and padding past the list's end
                 const int m = !more ? cnt[s] : (cnt[s] >= 32 ? cnt[s] & ~15 : 0);
-                if (lane < 16) W.list[s][cnt[s] + lane] = (unsigned)c.nr;
+                if (!EXACT && lane < 16) W.list[s][cnt[s] + lane] = (unsigned)c.nr;
                 if (lane == s) { W.cnt[s] = m; W.first[s] = cnt[s] - m; }
                 cnt[s] -= m;
             }
             __syncwarp();
+            if constexpr (EXACT) {
+#pragma unroll 1
+                for (int s = 0; s < NQ; ++s)
+                    w_dense_exact<G, IFACE, NP>(c, W, *X, iset, lane, s, W.first[s], W.cnt[s], gsum);
+            } else {
             auto lists = [&](auto elec, auto clash) {
 #pragma unroll 1
                 for (int s = 0; s < NQ; ++s)
@@ -773,6 +826,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
                 gsum.elec += r.elec;
                 gsum.vdw += r.vdw;
                 if (NP) gsum.np += r.np;
+            }
             }
             __syncwarp();
         } while (more);
@@ -809,10 +863,11 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
 // STAGE: the candidates reach shared memory by bulk copies (WStage) instead
 // of L1 loads (selected per context; the measured alternative)
 // NP: near pairs are counted (launches with parts)
-template <int G, bool IFACE, bool NP, bool STAGE = false>
-__global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchParams p) {
+// EXACT: f64 pair math in the reference's operation order
+template <int G, bool IFACE, bool NP, bool STAGE = false, bool EXACT = false>
+__global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCKS) k_score_warp(LaunchParams p) {
     static_assert(G == 4 || G == 8 || G == 16 || G == 32, "group size");
-    static_assert(!(STAGE && IFACE), "the staged variant is the plain kernel's");
+    static_assert(!(STAGE && (IFACE || EXACT)), "the staged variant is the plain kernel's");
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char wk_smem[];
     const int lane = w_lane();
@@ -822,6 +877,9 @@ __global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchPara
     WStage* S = STAGE ? reinterpret_cast<WStage*>(wk_smem + (WK_THREADS / 32) * (sizeof(WSlots<G>) + sizeof(ComplexDev))) +
                             (threadIdx.x >> 5)
                       : nullptr;
+    WExact<G>* X = EXACT ? reinterpret_cast<WExact<G>*>(wk_smem + (WK_THREADS / 32) * (sizeof(WSlots<G>) + sizeof(ComplexDev))) +
+                               (threadIdx.x >> 5)
+                         : nullptr;
     if (STAGE) {
         if (lane == 0) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(w_smem_u32(&S->bar)), "r"(1));
@@ -872,7 +930,8 @@ __global__ void __launch_bounds__(WK_THREADS, WK_BLOCKS) k_score_warp(LaunchPara
         if (lane == 0) W.part = p.sub ? p.partials + 4 * (first_part + g0) : nullptr;
         __syncwarp();
         WAcc acc;
-        w_groups<G, false, IFACE, NP, STAGE>(c, W, nullptr, nullptr, p.status, lane, g0, g1, 1, [](int k) { return k; }, acc, S);
+        w_groups<G, false, IFACE, NP, STAGE, EXACT>(c, W, nullptr, nullptr, p.status, lane, g0, g1, 1,
+                                                    [](int k) { return k; }, acc, S, X);
         if (IFACE && W.ibits) w_iface_flush(W, c);
         double* const pose_part = p.partials + 4 * first_part;
         if (!p.sub) {
@@ -1029,8 +1088,8 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
             }
             __syncthreads();
             // warp k scores the near groups k, k + NW, ...
-            w_groups<G, true, IFACE, NP>(c, W, D, &hash, p.status, lane, wid, total, NW,
-                                         [&](int k) { return g0 + s_list[k]; }, acc, nullptr, far_sep);
+            w_groups<G, true, IFACE, NP, false, false>(c, W, D, &hash, p.status, lane, wid, total, NW,
+                                         [&](int k) { return g0 + s_list[k]; }, acc, nullptr, nullptr, far_sep);
             if (g0 + WD_NEAR < ngrp) __syncthreads();   // the list is read
         }
         if (IFACE && W.ibits) w_iface_flush(W, c);   // before the block's barrier below
@@ -1078,7 +1137,7 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
 // per SM resident; here every thread has independent gathers in flight.
 // Skipped (masked) poses are left alone.
 constexpr int FAR_THREADS = 256;
-__global__ void __launch_bounds__(FAR_THREADS, 4) k_far_poses(LaunchParams p) {
+static __global__ void __launch_bounds__(FAR_THREADS, 4) k_far_poses(LaunchParams p) {
     __shared__ double s_red[4][32];
     for (long long w = blockIdx.x; w < p.total_work; w += gridDim.x) {
         const int b = find_item(p.item_work0, p.n_items, w);
