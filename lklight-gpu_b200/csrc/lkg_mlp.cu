@@ -1176,17 +1176,19 @@ int lkg_surrogate_create(lkg_ctx* ctx, int complex_id, uint64_t seed, lkg_surrog
     S->cid = complex_id;
     const ComplexRec& cr = *ctx->cx[complex_id];
     // anchors: 16 ligand atoms spread by farthest-point sampling over the
-    // (sorted) ligand reference coordinates
+    // ligand reference coordinates in group order (its first atom is the
+    // first anchor, ties go to the earlier one)
     const int nl = cr.d.nl;
-    std::vector<float4> lp(nl);
-    cudaMemcpy(lp.data(), cr.d.lpos, nl * sizeof(float4), cudaMemcpyDeviceToHost);
+    std::vector<float4> sorted(nl), lp(nl);
+    cudaMemcpy(sorted.data(), cr.d.lpos, nl * sizeof(float4), cudaMemcpyDeviceToHost);
+    for (int i = 0; i < nl; ++i) lp[i] = sorted[cr.lgroup_order[i]];
     std::vector<int> anc;
     std::vector<float> dmin(nl, 1e30f);
     int cur = 0;
     float rmax = 0.f;
     for (int i = 0; i < nl; ++i) rmax = std::max(rmax, std::sqrt(lp[i].x * lp[i].x + lp[i].y * lp[i].y + lp[i].z * lp[i].z));
     for (int a = 0; a < NA; ++a) {
-        anc.push_back(cur);
+        anc.push_back(cr.lgroup_order[cur]);
         int best = 0;
         float bd = -1.f;
         for (int i = 0; i < nl; ++i) {

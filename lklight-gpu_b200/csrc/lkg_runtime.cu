@@ -331,8 +331,13 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
     bisect_groups(L.c.data(), order.data(), n, ctx->group);
+    const std::vector<int> coarse = order;
     for (int k = 0; k < n; k += ctx->group)   // and quads compact inside each group
         bisect_groups(L.c.data(), order.data() + k, std::min(ctx->group, n - k), 4);
+    std::vector<int> at(n);
+    for (int k = 0; k < n; ++k) at[order[k]] = k;
+    cr.lgroup_order.resize(n);
+    for (int k = 0; k < n; ++k) cr.lgroup_order[k] = at[coarse[k]];
     std::vector<float4> pos(n), par(n);
     std::vector<float2> sol(n);
     std::vector<double4> pos64(n), par64(n);

@@ -82,6 +82,10 @@ struct ComplexRec {
     DBuf rpos, rpar, rpk, rsolv, rpos64, rpar64, rsolv64, rorig, cell_start;
     DBuf rlb;   // distance lower bound of the receptor (ComplexDev::rlb)
     DBuf lpos, lpar, lsolv, lpos64, lpar64, lsolv64, lorig, lgrp, lquad;
+    // the ligand's atoms (kernel indices) in the order of the bisection into
+    // groups, before each group was bisected into quads: the surrogate's
+    // anchors are sampled in this order
+    std::vector<int> lgroup_order;
     DBuf phi;
     DBuf rtag, ltag;   // interface tags (restraints / membrane), when set
     ComplexDev d{};
