@@ -38,6 +38,17 @@ namespace mlp {
 
 constexpr int IN = 64, H = 256, NA = 16;   // features, width, anchors
 
+// Programmatic dependent launch.  The kernels of a training step and of a
+// prediction are 3-10 us each and follow one another, so a third of a step was
+// launch gaps and prologues.  Each kernel touches global memory only after its
+// predecessor has finished (pdl_wait) and then lets its successor start
+// (pdl_trigger); every kernel waits, so the order of all memory accesses is
+// that of the stream.  Without the launch attribute both are no-ops.  A step
+// at batch 1024: 70 us as plain graph nodes, 65 so; 76 when the successors
+// were let in before the wait (several kernels deep).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // features
 // ---------------------------------------------------------------------------
@@ -55,6 +66,8 @@ struct TargetArgs {
 __global__ void k_features(const ComplexDev* __restrict__ cxs, int cid, const double* __restrict__ poses, int n,
                            const int* __restrict__ anchors, float tscale, __nv_bfloat16* __restrict__ feat,
                            TargetArgs tgt) {
+    pdl_wait();
+    pdl_trigger();
     const ComplexDev& c = cxs[cid];
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int pose = t / NA, a = t % NA;
@@ -246,17 +259,18 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 
 // TN: output columns of a CTA (256, or 128 with blockIdx.y picking the half
 // when the row tiles alone would leave most SMs idle)
+// One CTA's tile (bx: row tile, by: column tile); a body of its own so that a
+// kernel can run it beside other blocks.
 template <int EPI, int TN>
-__global__ void __launch_bounds__(128, 1)
-k_gemm_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int M, int K,
-          const float* __restrict__ bias, const __nv_bfloat16* __restrict__ Hm, __nv_bfloat16* __restrict__ Y,
-          int* __restrict__ status) {
+__device__ __forceinline__ void gemm_tc_block(const CUtensorMap& mapA, const CUtensorMap& mapB, int M, int K,
+                                              const float* __restrict__ bias, const __nv_bfloat16* __restrict__ Hm,
+                                              __nv_bfloat16* __restrict__ Y, int* __restrict__ status, int bx, int by) {
     static_assert(TN == 128 || TN == 256, "tile width");
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     __shared__ __align__(8) unsigned long long bars[2];   // operands loaded, accumulator ready
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * TC_BM, n0 = blockIdx.y * TN, nslab = K / TC_KS;
+    const int m0 = bx * TC_BM, n0 = by * TN, nslab = K / TC_KS;
     const uint32_t base = (smem_u32(tc_smem) + 1023u) & ~1023u;   // SW128 atoms are 1024-byte aligned
     const uint32_t sA = base, sB = base + (uint32_t)(nslab * TC_BM * 128);
     const uint32_t bar_ld = smem_u32(&bars[0]), bar_mma = smem_u32(&bars[1]);
@@ -270,6 +284,10 @@ k_gemm_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar_ld), "r"(1));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar_mma), "r"(1));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (tid == 0) {
         const uint32_t bytes = (uint32_t)(nslab * (TC_BM + TN) * 128);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar_ld), "r"(bytes) : "memory");
         for (int sl = 0; sl < nslab; ++sl) {
@@ -360,6 +378,14 @@ k_gemm_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
     }
 }
 
+template <int EPI, int TN>
+__global__ void __launch_bounds__(128, 1)
+k_gemm_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int M, int K,
+          const float* __restrict__ bias, const __nv_bfloat16* __restrict__ Hm, __nv_bfloat16* __restrict__ Y,
+          int* __restrict__ status) {
+    gemm_tc_block<EPI, TN>(mapA, mapB, M, K, bias, Hm, Y, status, blockIdx.x, blockIdx.y);
+}
+
 // ---------------------------------------------------------------------------
 // Forward layer for large predictions: a persistent, warp-specialised
 // tcgen05 GEMM.  Each CTA (one per SM) keeps the layer's weights B
@@ -427,6 +453,8 @@ k_gemm_tc_pp(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&bfull)), "r"(1));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    pdl_wait();
+    pdl_trigger();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -581,6 +609,7 @@ k_gemm_tc_pp(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
 constexpr int TCW_ROWS = 128;                       // batch rows per CTA (two 64-row slabs)
 constexpr int TCW_SLAB = 64;                        // batch rows per TMA box
 constexpr size_t TCW_SMEM = (size_t)(TC_BM + TC_N) * TCW_ROWS * 2 + 1024;
+constexpr size_t BWD_SMEM = TCW_SMEM > TC_SMEM ? TCW_SMEM : TC_SMEM;
 
 __device__ __forceinline__ uint64_t tc_desc_mn(uint32_t saddr, uint32_t lbo_bytes) {
     return (uint64_t)((saddr >> 4) & 0x3fff) | ((uint64_t)((lbo_bytes >> 4) & 0x3fff) << 16) |
@@ -588,9 +617,8 @@ __device__ __forceinline__ uint64_t tc_desc_mn(uint32_t saddr, uint32_t lbo_byte
 }
 
 template <int TN>
-__global__ void __launch_bounds__(128, 1)
-k_wgrad_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int rows,
-           float* __restrict__ part, int* __restrict__ status) {
+__device__ __forceinline__ void wgrad_tc_block(const CUtensorMap& mapA, const CUtensorMap& mapB, int rows,
+                                               float* __restrict__ part, int* __restrict__ status, int bx, int by) {
     static_assert(TN == 64 || TN == 256, "input width");
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     __shared__ __align__(8) unsigned long long bars[2];
@@ -598,7 +626,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     constexpr int NSLAB = TCW_ROWS / TCW_SLAB;
     constexpr uint32_t A_SLAB = TC_BM * TCW_SLAB * 2, B_SLAB = TN * TCW_SLAB * 2;   // bytes per slab
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * TC_BM, r0 = blockIdx.y * TCW_ROWS;
+    const int m0 = bx * TC_BM, r0 = by * TCW_ROWS;
     const uint32_t base = (smem_u32(tc_smem) + 1023u) & ~1023u;
     const uint32_t sA = base, sB = base + (uint32_t)NSLAB * A_SLAB;
     const uint32_t bar_ld = smem_u32(&bars[0]), bar_mma = smem_u32(&bars[1]);
@@ -611,6 +639,10 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar_ld), "r"(1));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar_mma), "r"(1));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (tid == 0) {
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
                      :: "r"(bar_ld), "r"((uint32_t)NSLAB * (A_SLAB + B_SLAB)) : "memory");
         // slab sl: A boxes of 64 output rows (o) and B boxes of 64 inputs (i),
@@ -652,7 +684,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
         if (lane == 0) atomicOr(status, 4);
     } else {
         // warp w: output rows o = m0 + 32 w + lane (TMEM lanes), 32 columns at a time
-        float* out = part + (size_t)blockIdx.y * H * TN + (size_t)(m0 + warp * 32 + lane) * TN;
+        float* out = part + (size_t)by * H * TN + (size_t)(m0 + warp * 32 + lane) * TN;
         for (int cl = 0; cl < TN; cl += 32) {
             uint32_t r[32];
             const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)cl;
@@ -683,9 +715,33 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     }
 }
 
+template <int TN>
+__global__ void __launch_bounds__(128, 1)
+k_wgrad_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int rows,
+           float* __restrict__ part, int* __restrict__ status) {
+    wgrad_tc_block<TN>(mapA, mapB, rows, part, status, blockIdx.x, blockIdx.y);
+}
+
+// The weight gradient of a layer and its backward-data product (EPI_BWD, 128
+// columns a CTA) read the same dC and write apart: one launch for both, so a
+// training step is a chain of 8 launches instead of 11 (the chain, not the
+// work, is what a step of 1024 rows costs).  Blocks 0 .. 2 splits - 1: the
+// weight gradient; the others: the product.
+__global__ void __launch_bounds__(128, 1)
+k_bwd_pair(const __grid_constant__ CUtensorMap dcT, const __grid_constant__ CUtensorMap ain,
+           const __grid_constant__ CUtensorMap dc, const __grid_constant__ CUtensorMap w, int rows, int splits,
+           float* __restrict__ part, const __nv_bfloat16* __restrict__ Hm, __nv_bfloat16* __restrict__ Y,
+           int* __restrict__ status) {
+    const int nw = (H / TC_BM) * splits, b = blockIdx.x;
+    if (b < nw) wgrad_tc_block<H>(dcT, ain, rows, part, status, b % (H / TC_BM), b / (H / TC_BM));
+    else gemm_tc_block<EPI_BWD, 128>(dc, w, rows, H, nullptr, Hm, Y, status, (b - nw) >> 1, (b - nw) & 1);
+}
+
 // last layer: y[n] = H3[n] . w3 + b3
 __global__ void k_head(const __nv_bfloat16* __restrict__ H3, int n, const float* __restrict__ w3, const float* b3,
                        float* __restrict__ y) {
+    pdl_wait();
+    pdl_trigger();
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= n) return;
     float s = 0.f;
@@ -712,6 +768,8 @@ __global__ void __launch_bounds__(H) k_loss_head(const float* __restrict__ t, co
     static_assert(RL % (H / 32) == 0, "whole rows per warp");
     __shared__ float s_y[RL];
     const int k = threadIdx.x, r0 = blockIdx.x * RL, r1 = min(n, r0 + RL);
+    pdl_wait();
+    pdl_trigger();
     for (int rr = k >> 5; rr < RL; rr += H / 32) {
         const int row = r0 + rr, lane = k & 31;
         if (row < r1) {
@@ -748,12 +806,29 @@ struct ColSums {
     const __nv_bfloat16* dC[3];
     float* part;
 };
-__global__ void __launch_bounds__(H) k_colsum3(ColSums a, int n) {
-    const int col = threadIdx.x, blk = blockIdx.x, L = blockIdx.y, r0 = blk * RB, r1 = min(n, r0 + RB);
+__device__ __forceinline__ void colsum_block(const ColSums& a, int n, int nblk, int blk, int L) {
+    const int r0 = blk * RB, r1 = min(n, r0 + RB);
     const __nv_bfloat16* dC = a.dC[L];
-    float s = 0.f;
-    for (int r = r0; r < r1; ++r) s += __bfloat162float(dC[(size_t)r * H + col]);
-    a.part[((size_t)L * gridDim.x + blk) * H + col] = s;
+    pdl_wait();
+    pdl_trigger();
+    for (int col = threadIdx.x; col < H; col += blockDim.x) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int r = r0; r < r1; ++r) s += __bfloat162float(dC[(size_t)r * H + col]);
+        a.part[((size_t)L * nblk + blk) * H + col] = s;
+    }
+}
+__global__ void __launch_bounds__(H) k_colsum3(ColSums a, int n) {
+    colsum_block(a, n, gridDim.x, blockIdx.x, blockIdx.y);
+}
+// the first layer's weight gradient (blocks 0 .. 2 splits - 1) and the bias
+// partials of all layers (the others) in one launch, as k_bwd_pair
+__global__ void __launch_bounds__(128, 1)
+k_wgrad0_colsum3(const __grid_constant__ CUtensorMap dcT, const __grid_constant__ CUtensorMap ain, int rows, int splits,
+                 float* __restrict__ part, int* __restrict__ status, ColSums a, int nblk) {
+    const int nw = (H / TC_BM) * splits, b = blockIdx.x;
+    if (b < nw) wgrad_tc_block<IN>(dcT, ain, rows, part, status, b % (H / TC_BM), b / (H / TC_BM));
+    else colsum_block(a, rows, nblk, (b - nw) % nblk, (b - nw) / nblk);
 }
 
 // the three GEMM layers inside the flat parameter vector
@@ -786,6 +861,8 @@ __global__ void k_grad_adam(float* __restrict__ p, float* __restrict__ gr, float
                             int* __restrict__ step, AdamLayers L, GradSums G, int apply) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float t = 0.f;
+    pdl_wait();
+    pdl_trigger();
     if (apply) {
         t = (float)*reinterpret_cast<volatile int*>(step);
         __syncthreads();
@@ -865,6 +942,7 @@ using namespace lkg::mlp;
 struct lkg_surrogate {
     lkg_ctx* ctx = nullptr;
     int cid = -1;
+    bool pdl = false;   // the next launch follows a kernel of this file (programmatic dependent launch)
     float tscale = 50.f;
     float t_mu = 0.f, t_sd = 1.f, e_scale = 100.f;   // target standardisation
     DBuf anchors;
@@ -944,6 +1022,24 @@ cudaError_t gemm(cudaStream_t s, int M, int N, int K, const __nv_bfloat16* A, in
     return cudaGetLastError();
 }
 
+// a launch that may start while the kernel before it on the stream finishes
+// (S->pdl; off where that is not a kernel of this file)
+template <class... P, class... A>
+cudaError_t launch(lkg_surrogate* S, void (*kern)(P...), dim3 grid, int threads, size_t smem, A... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = S->ctx->stream;
+    cfg.attrs = at;
+    cfg.numAttrs = S->pdl ? 1 : 0;
+    S->pdl = true;
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 float* P(lkg_surrogate* S, int k) { return S->p.as<float>() + S->off[k]; }
 // layer L's region of the weight-gradient partials (layers 0, 1, 2 in turn)
 float* wpart_of(lkg_surrogate* S, int L) {
@@ -986,9 +1082,8 @@ cudaError_t gemm_tc(lkg_surrogate* S, int n, int K, const __nv_bfloat16* A, cons
         if (!tc_map(&ma, A, n, K, TC_BM) || !tc_map(&mb, B, TC_N, K, TC_N)) return cudaErrorInvalidValue;
         cudaError_t e = cudaFuncSetAttribute(k_gemm_tc_pp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PP_SMEM);
         if (e != cudaSuccess) return e;
-        k_gemm_tc_pp<<<S->ctx->sm_count, PP_THREADS, PP_SMEM, S->ctx->stream>>>(ma, mb, n, K, b, Y,
-                                                                              S->d_status.as<int>());
-        return cudaGetLastError();
+        return launch(S, k_gemm_tc_pp, dim3(S->ctx->sm_count), PP_THREADS, PP_SMEM, ma, mb, n, K, b, Y,
+                      S->d_status.as<int>());
     }
     // few row tiles (training batches): two CTAs of 128 columns per tile
     const bool split = 2 * tiles <= S->ctx->sm_count;
@@ -999,8 +1094,7 @@ cudaError_t gemm_tc(lkg_surrogate* S, int n, int K, const __nv_bfloat16* A, cons
     auto kern = split ? k_gemm_tc<EPI, 128> : k_gemm_tc<EPI, 256>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
     if (e != cudaSuccess) return e;
-    kern<<<dim3(tiles, TC_N / tn), 128, TC_SMEM, S->ctx->stream>>>(ma, mb, n, K, b, Hm, Y, S->d_status.as<int>());
-    return cudaGetLastError();
+    return launch(S, kern, dim3(tiles, TC_N / tn), 128, TC_SMEM, ma, mb, n, K, b, Hm, Y, S->d_status.as<int>());
 }
 
 // dW[H x kin] partials: part[split][o][i] = sum over the split's batch rows r
@@ -1015,8 +1109,7 @@ cudaError_t wgrad_tc(lkg_surrogate* S, int n, int kin, const __nv_bfloat16* dC, 
     auto kern = kin == H ? k_wgrad_tc<256> : k_wgrad_tc<64>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TCW_SMEM);
     if (e != cudaSuccess) return e;
-    kern<<<dim3(H / TC_BM, splits), 128, TCW_SMEM, S->ctx->stream>>>(ma, mb, n, part, S->d_status.as<int>());
-    return cudaGetLastError();
+    return launch(S, kern, dim3(H / TC_BM, splits), 128, TCW_SMEM, ma, mb, n, part, S->d_status.as<int>());
 }
 
 // forward of n feature rows (X, default S->X): H1..H3, and with `head`
@@ -1041,8 +1134,8 @@ int forward(lkg_surrogate* S, int n, const __nv_bfloat16* X = nullptr, bool head
     }
     S->ctx->launches += 3;
     if (head) {
-        k_head<<<(n + 7) / 8, 256, 0, s>>>(S->H3.as<__nv_bfloat16>(), n, P(S, 6), P(S, 7), S->y.as<float>());
-        LKG_CK(cudaGetLastError(), "mlp head");
+        LKG_CK(launch(S, k_head, dim3((n + 7) / 8), 256, 0, S->H3.as<__nv_bfloat16>(), n, P(S, 6), P(S, 7),
+                      S->y.as<float>()), "mlp head");
         S->ctx->launches += 1;
     }
     return 0;
@@ -1059,12 +1152,36 @@ int backward(lkg_surrogate* S, int n, const __nv_bfloat16* X = nullptr, const fl
     if (!X) X = S->X.as<__nv_bfloat16>();
     if (!t) t = S->t.as<float>();
     const int nlblk = (n + RL - 1) / RL;
-    k_loss_head<<<nlblk, H, 0, s>>>(t, S->H3.as<__nv_bfloat16>(), n, P(S, 6), P(S, 7), S->y.as<float>(),
-                                    S->dH3.as<__nv_bfloat16>(), S->rpart.as<float>());
-    LKG_CK(cudaGetLastError(), "mlp loss");
+    LKG_CK(launch(S, k_loss_head, dim3(nlblk), H, 0, t, S->H3.as<__nv_bfloat16>(), n, P(S, 6), P(S, 7), S->y.as<float>(),
+                  S->dH3.as<__nv_bfloat16>(), S->rpart.as<float>()), "mlp loss");
     const int splits = wgrad_splits(n);
     const __nv_bfloat16* acts[3] = {S->H1.as<__nv_bfloat16>(), S->H2.as<__nv_bfloat16>(), S->H3.as<__nv_bfloat16>()};
     __nv_bfloat16* dacts[3] = {S->dH1.as<__nv_bfloat16>(), S->dH2.as<__nv_bfloat16>(), S->dH3.as<__nv_bfloat16>()};
+    const ColSums cs{{S->dH1.as<__nv_bfloat16>(), S->dH2.as<__nv_bfloat16>(), S->dH3.as<__nv_bfloat16>()},
+                     S->cpart.as<float>()};
+    if (S->tc && 2 * ((n + TC_BM - 1) / TC_BM) <= S->ctx->sm_count) {
+        // training batches (where the products run as 128-column CTAs)
+        const int nz = (n + TCW_ROWS - 1) / TCW_ROWS, tiles = (n + TC_BM - 1) / TC_BM, nblk = (n + RB - 1) / RB;
+        LKG_CK(cudaFuncSetAttribute(k_bwd_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BWD_SMEM), "mlp bwd");
+        LKG_CK(cudaFuncSetAttribute(k_wgrad0_colsum3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TCW_SMEM), "mlp bwd");
+        for (int L = 2; L >= 0; --L) {
+            S->wnz[L] = nz;
+            alignas(64) CUtensorMap dct, ain, dc, w;
+            if (!tc_map(&dct, dacts[L], n, H, TCW_SLAB) || !tc_map(&ain, L ? acts[L - 1] : X, n, L ? H : IN, TCW_SLAB))
+                return set_error(LKG_ERR_LAUNCH, "mlp bwd tensor maps");
+            if (L == 0) {
+                LKG_CK(launch(S, k_wgrad0_colsum3, dim3((H / TC_BM) * nz + 3 * nblk), 128, TCW_SMEM, dct, ain, n, nz,
+                              wpart_of(S, 0), S->d_status.as<int>(), cs, nblk), "mlp wgrad and bias grad");
+                break;
+            }
+            if (!tc_map(&dc, dacts[L], n, H, TC_BM) || !tc_map(&w, S->w[L].p, TC_N, H, 128))
+                return set_error(LKG_ERR_LAUNCH, "mlp bwd tensor maps");
+            LKG_CK(launch(S, k_bwd_pair, dim3((H / TC_BM) * nz + 2 * tiles), 128, BWD_SMEM, dct, ain, dc, w, n, nz,
+                          wpart_of(S, L), acts[L - 1], dacts[L - 1], S->d_status.as<int>()), "mlp bwd");
+        }
+        S->ctx->launches += 4;   // head and loss, 2 x (weight gradient and backward data), the rest
+        return 0;
+    }
     for (int L = 2; L >= 0; --L) {
         const int kin = L == 0 ? IN : H;
         const __nv_bfloat16* ain = L == 0 ? X : acts[L - 1];
@@ -1088,10 +1205,7 @@ int backward(lkg_surrogate* S, int n, const __nv_bfloat16* X = nullptr, const fl
                                                     dacts[L - 1], H, nullptr, acts[L - 1])), "mlp bwd");
         }
     }
-    const ColSums cs{{S->dH1.as<__nv_bfloat16>(), S->dH2.as<__nv_bfloat16>(), S->dH3.as<__nv_bfloat16>()},
-                     S->cpart.as<float>()};
-    k_colsum3<<<dim3((n + RB - 1) / RB, 3), H, 0, s>>>(cs, n);
-    LKG_CK(cudaGetLastError(), "mlp bias grad");
+    LKG_CK(launch(S, k_colsum3, dim3((n + RB - 1) / RB, 3), H, 0, cs, n), "mlp bias grad");
     S->ctx->launches += 7;   // head and loss, 3 x weight-gradient partials, 2 x backward data, bias partials
     return 0;
 }
@@ -1118,10 +1232,8 @@ int grad_step(lkg_surrogate* S, int n, bool apply, float lr = 0.f) {
     G.nlblk = (n + RL - 1) / RL;
     G.loss = S->loss.as<float>();
     const int np = (int)NPARAM;
-    k_grad_adam<<<(np + 255) / 256, 256, 0, s>>>(S->p.as<float>(), S->g.as<float>(), S->m1.as<float>(),
-                                                 S->m2.as<float>(), np, lr, b1, b2, eps, S->d_step.as<int>(), L, G,
-                                                 apply ? 1 : 0);
-    LKG_CK(cudaGetLastError(), "mlp grad / adam");
+    LKG_CK(launch(S, k_grad_adam, dim3((np + 255) / 256), 256, 0, S->p.as<float>(), S->g.as<float>(), S->m1.as<float>(),
+                  S->m2.as<float>(), np, lr, b1, b2, eps, S->d_step.as<int>(), L, G, apply ? 1 : 0), "mlp grad / adam");
     S->ctx->launches += 1;
     return 0;
 }
@@ -1149,9 +1261,9 @@ int features(lkg_surrogate* S, int n, const double* d_poses, const double* d_sco
     if (!t_out) t_out = S->t.as<float>();
     const int threads = 256, blocks = (int)(((size_t)n * NA + threads - 1) / threads);
     const TargetArgs tgt{d_scores, S->e_scale, S->t_mu, S->t_sd, d_scores ? t_out : nullptr};
-    k_features<<<blocks, threads, 0, S->ctx->stream>>>(S->ctx->d_cx.as<ComplexDev>(), S->cid, d_poses, n,
-                                                       S->anchors.as<int>(), S->tscale, X_out, tgt);
-    LKG_CK(cudaGetLastError(), "features");
+    S->pdl = false;   // what precedes on the stream is the caller's
+    LKG_CK(launch(S, k_features, dim3(blocks), threads, 0, S->ctx->d_cx.as<ComplexDev>(), S->cid, d_poses, n,
+                  S->anchors.as<int>(), S->tscale, X_out, tgt), "features");
     S->ctx->launches++;
     return 0;
 }
@@ -1159,6 +1271,8 @@ int features(lkg_surrogate* S, int n, const double* d_poses, const double* d_sco
 // predictions back to score units: the inverse of the standardised target
 // t = (asinh(score / e_scale) - mu) / sd that k_features writes in training
 __global__ void k_untarget(const float* __restrict__ y, int n, float e_scale, float mu, float sd, double* __restrict__ out) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = (double)(sinhf(y[i] * sd + mu) * e_scale);
 }
@@ -1283,9 +1397,8 @@ int lkg_surrogate_predict(lkg_surrogate* S, int n, const double* d_poses, double
         const int m = std::min(PRED_CHUNK, n - b0);
         if ((st = features(S, m, d_poses + 7 * (size_t)b0))) return st;
         if ((st = forward(S, m))) return st;
-        k_untarget<<<(m + 255) / 256, 256, 0, S->ctx->stream>>>(S->y.as<float>(), m, S->e_scale, S->t_mu, S->t_sd,
-                                                                d_pred + b0);
-        LKG_CK(cudaGetLastError(), "predict");
+        LKG_CK(launch(S, k_untarget, dim3((m + 255) / 256), 256, 0, S->y.as<float>(), m, S->e_scale, S->t_mu, S->t_sd,
+                      d_pred + b0), "predict");
         S->ctx->launches++;
     }
     return set_ok();
@@ -1318,7 +1431,7 @@ int lkg_surrogate_train(lkg_surrogate* S, int n, const double* d_poses, const do
     // the features and targets of the whole set, once (they do not change
     // between epochs); then one epoch = per batch the forward layers, the
     // backward and one gradient / Adam launch (the loss is summed on the
-    // device), captured once in a CUDA graph and replayed `epochs` times
+    // device), for long trainings captured once in a CUDA graph and replayed
     if (n > S->cap_tr) {
         LKG_CK(S->Xtr.reserve((size_t)n * IN * sizeof(__nv_bfloat16)), "surrogate alloc");
         LKG_CK(S->ttr.reserve((size_t)n * sizeof(float)), "surrogate alloc");
@@ -1329,6 +1442,7 @@ int lkg_surrogate_train(lkg_surrogate* S, int n, const double* d_poses, const do
     if ((st = features(S, n, d_poses, d_scores, Xtr, ttr))) return st;
     auto epoch = [&]() -> int {
         LKG_CK(cudaMemsetAsync(S->loss.p, 0, sizeof(float), s), "mlp loss clear");
+        S->pdl = false;   // not after a memset
         for (int b0 = 0; b0 + batch <= n; b0 += batch) {
             const __nv_bfloat16* xb = Xtr + (size_t)b0 * IN;
             int r;
@@ -1338,10 +1452,13 @@ int lkg_surrogate_train(lkg_surrogate* S, int n, const double* d_poses, const do
         }
         return 0;
     };
+    constexpr int GRAPH_EPOCHS = 16;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     bool graphed = false;
-    if (epochs > 1 && cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+    // (capturing and instantiating 64 to 88 launches costs 0.4 ms and saves
+    // some 25 us an epoch over plain launches, so short trainings go without)
+    if (epochs >= GRAPH_EPOCHS && cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
         const int r = epoch();
         const cudaError_t e = cudaStreamEndCapture(s, &graph);
         if (r) { if (graph) cudaGraphDestroy(graph); return r; }
@@ -1416,6 +1533,7 @@ int lkg_surrogate_grad(lkg_surrogate* S, int n, const uint16_t* feats, const flo
     LKG_CK(cudaMemcpy(S->X.p, feats, (size_t)n * IN * 2, cudaMemcpyHostToDevice), "grad upload");
     LKG_CK(cudaMemcpy(S->t.p, targets, (size_t)n * 4, cudaMemcpyHostToDevice), "grad upload");
     LKG_CK(cudaMemsetAsync(S->loss.p, 0, sizeof(float), S->ctx->stream), "grad loss clear");
+    S->pdl = false;
     int st;
     if ((st = forward(S, n, nullptr, false)) || (st = backward(S, n)) || (st = grad_step(S, n, false))) return st;
     LKG_CK(cudaStreamSynchronize(S->ctx->stream), "grad");
