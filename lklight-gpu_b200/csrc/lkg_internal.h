@@ -116,6 +116,7 @@ struct LaunchParams {
     int* pose_counter;           // [N]
     unsigned long long* work_counter;  // [2]: next unit, CTAs done
     int* status;                 // [4]: error flags (capacity overflow, bad index)
+    int* host_status;            // optional, page-locked host: the launch's last block leaves status[0] here
     int max_tiles;               // unused by the kernels (kept for layout)
     // per-atom outputs (cuda_full_score): pose 0 of item 0, caller atom order
     float* atom_elec;

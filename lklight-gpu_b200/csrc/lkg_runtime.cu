@@ -719,7 +719,7 @@ size_t group_spill_bytes(lkg_ctx* ctx, const Group& G, bool exact) {
 
 int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, const double* d_poses,
                  double* d_scores, double* d_parts, int raw_pairs, int solv_only, float* atom_e, float* atom_v,
-                 const unsigned char* pose_mask, double* d_iface) {
+                 const unsigned char* pose_mask, double* d_iface, int* host_status) {
     const bool exact = ctx->precision == LKG_PREC_EXACT;
     const int ni = (int)G.ic.size();
     LaunchParams p{};
@@ -744,6 +744,7 @@ int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, cons
     p.pose_counter = sc.pose_counter.as<int>();
     p.work_counter = sc.work_counter.as<unsigned long long>();
     p.status = sc.status.as<int>();
+    p.host_status = host_status;
     p.max_tiles = 0;
     p.atom_elec = atom_e;
     p.atom_vdw = atom_v;
@@ -798,7 +799,7 @@ int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, cons
 
 int launch_items(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, const double* d_poses,
                  double* d_scores, double* d_parts, int raw_pairs, int solv_only, float* atom_e,
-                 float* atom_v, double* d_iface) {
+                 float* atom_v, double* d_iface, int* host_status) {
     if (n_items <= 0) return set_ok();
     Group g[2];
     size_t n_poses = 0;
@@ -825,7 +826,7 @@ int launch_items(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, c
     for (int k = 0; k < 2; ++k) {
         if (g[k].ic.empty()) continue;
         st = launch_group(ctx, g[k], ctx->d_items.as<char>() + (k ? b0 : 0), ctx->scratch, d_poses, d_scores, d_parts,
-                          raw_pairs, solv_only, atom_e, atom_v, nullptr, d_iface);
+                          raw_pairs, solv_only, atom_e, atom_v, nullptr, d_iface, host_status);
         if (st) return st;
     }
     return set_ok();
@@ -867,6 +868,18 @@ int check_status_word(int* d_status) {
 }
 
 int check_status(lkg_ctx* ctx) { return check_status_word(ctx->scratch.status.as<int>()); }
+
+cudaError_t status_word(lkg_ctx* ctx, int** word) {
+    const cudaError_t e = ctx->h_status.reserve(64);
+    if (e != cudaSuccess) return e;
+    *word = ctx->h_status.as<int>();
+    **word = 0;
+    return cudaSuccess;
+}
+
+int check_status_seen(lkg_ctx* ctx, const int* word) {
+    return *reinterpret_cast<const volatile int*>(word) ? check_status(ctx) : set_ok();
+}
 
 }  // namespace lkg
 
@@ -1083,14 +1096,32 @@ static int score_host(lkg_ctx* ctx, int id, int n, const double* poses, double* 
     LKG_CK(ctx->h_poses.reserve(pb), "staging");
     LKG_CK(ctx->h_out.reserve(ob + qb + ib), "staging");
     LKG_CK(ctx->d_poses.reserve(pb), "staging");
-    LKG_CK(ctx->d_scores.reserve(ob), "staging");
-    LKG_CK(ctx->d_parts.reserve(qb + ib), "staging");
+    int* status = nullptr;
+    LKG_CK(status_word(ctx, &status), "staging");
     memcpy(ctx->h_poses.p, poses, pb);
     LKG_CK(cudaMemcpyAsync(ctx->d_poses.p, ctx->h_poses.p, pb, cudaMemcpyHostToDevice, ctx->stream), "pose upload");
+    int st;
+    if (n <= HOST_WRITE_POSES) {
+        double* h_scores = ctx->h_out.as<double>();
+        double* h_parts = (double*)(ctx->h_out.as<char>() + ob);
+        double* h_iface = (double*)(ctx->h_out.as<char>() + ob + qb);
+        if (iface) memset(h_iface, 0, ib);   // zeros for a complex without restraints
+        if ((st = launch_items(ctx, 1, &id, &n, ctx->d_poses.as<double>(), h_scores, parts ? h_parts : nullptr, 0, 0,
+                               nullptr, nullptr, iface ? h_iface : nullptr, status)))
+            return st;
+        if ((st = wait_stream(ctx, 300.0))) return st;
+        if ((st = check_status_seen(ctx, status))) return st;
+        memcpy(scores, h_scores, ob);
+        if (parts) memcpy(parts, h_parts, qb);
+        if (iface) memcpy(iface, h_iface, ib);
+        return set_ok();
+    }
+    LKG_CK(ctx->d_scores.reserve(ob), "staging");
+    LKG_CK(ctx->d_parts.reserve(qb + ib), "staging");
     double* d_iface = iface ? (double*)(ctx->d_parts.as<char>() + qb) : nullptr;
     if (iface) LKG_CK(cudaMemsetAsync(d_iface, 0, ib, ctx->stream), "interface output");
-    int st = launch_items(ctx, 1, &id, &n, ctx->d_poses.as<double>(), ctx->d_scores.as<double>(),
-                          parts ? ctx->d_parts.as<double>() : nullptr, 0, 0, nullptr, nullptr, d_iface);
+    st = launch_items(ctx, 1, &id, &n, ctx->d_poses.as<double>(), ctx->d_scores.as<double>(),
+                      parts ? ctx->d_parts.as<double>() : nullptr, 0, 0, nullptr, nullptr, d_iface, status);
     if (st) return st;
     LKG_CK(cudaMemcpyAsync(ctx->h_out.p, ctx->d_scores.p, ob, cudaMemcpyDeviceToHost, ctx->stream), "score readback");
     if (parts)
@@ -1100,7 +1131,7 @@ static int score_host(lkg_ctx* ctx, int id, int n, const double* poses, double* 
         LKG_CK(cudaMemcpyAsync(ctx->h_out.as<char>() + ob + qb, d_iface, ib, cudaMemcpyDeviceToHost, ctx->stream),
                "interface readback");
     if ((st = wait_stream(ctx, 300.0))) return st;
-    if ((st = check_status(ctx))) return st;
+    if ((st = check_status_seen(ctx, status))) return st;
     memcpy(scores, ctx->h_out.p, ob);
     if (parts) memcpy(parts, ctx->h_out.as<char>() + ob, qb);
     if (iface) memcpy(iface, ctx->h_out.as<char>() + ob + qb, ib);
@@ -1153,8 +1184,10 @@ int lkg_score_multi(lkg_ctx* ctx, int n_items, const int* ids, const int* counts
         src = ctx->h_poses.as<double>();
     }
     LKG_CK(cudaMemcpyAsync(ctx->d_poses.p, src, pb, cudaMemcpyHostToDevice, ctx->stream), "pose upload");
+    int* status = nullptr;
+    LKG_CK(status_word(ctx, &status), "staging");
     int st = launch_items(ctx, n_items, ids, counts, ctx->d_poses.as<double>(), ctx->d_scores.as<double>(),
-                          parts ? ctx->d_parts.as<double>() : nullptr, 0, 0, nullptr, nullptr);
+                          parts ? ctx->d_parts.as<double>() : nullptr, 0, 0, nullptr, nullptr, nullptr, status);
     if (st) return st;
     double* dst_s = scores;
     double* dst_p = parts;
@@ -1166,7 +1199,7 @@ int lkg_score_multi(lkg_ctx* ctx, int n_items, const int* ids, const int* counts
     LKG_CK(cudaMemcpyAsync(dst_s, ctx->d_scores.p, ob, cudaMemcpyDeviceToHost, ctx->stream), "score readback");
     if (parts) LKG_CK(cudaMemcpyAsync(dst_p, ctx->d_parts.p, qb, cudaMemcpyDeviceToHost, ctx->stream), "parts readback");
     if ((st = wait_stream(ctx, 300.0))) return st;
-    if ((st = check_status(ctx))) return st;
+    if ((st = check_status_seen(ctx, status))) return st;
     if (!pin_out) {
         memcpy(scores, dst_s, ob);
         if (parts) memcpy(parts, dst_p, qb);

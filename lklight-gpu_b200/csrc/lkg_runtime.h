@@ -151,7 +151,7 @@ struct lkg_ctx {
     std::vector<char> last_items;   // tables currently in d_items
     // host-buffer call staging
     lkg::DBuf d_poses, d_scores, d_parts;
-    lkg::HBuf h_poses, h_out;
+    lkg::HBuf h_poses, h_out, h_status;
     int64_t launches = 0;
     lkg::Occupancy occ_tiles[2], occ_desolv[2];
     bool noalloc_used = false;      // lkg_score_device_noalloc ran on this context (its status word is checked)
@@ -186,9 +186,19 @@ int complex_set_restraints(lkg_ctx* ctx, int id, const int32_t* rres, int nres_r
 // one persistent launch group over items; device pointers
 int launch_items(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, const double* d_poses,
                  double* d_scores, double* d_parts, int raw_pairs, int solv_only, float* atom_e,
-                 float* atom_v, double* d_iface = nullptr);
+                 float* atom_v, double* d_iface = nullptr, int* host_status = nullptr);
 int wait_stream(lkg_ctx* ctx, double timeout_s);
 int check_status(lkg_ctx* ctx);
+// Poses up to which a host-buffer call lets the kernels write results and the
+// status word straight into page-locked host memory (8 bytes at a time over
+// PCIe, while the launch runs).  A one-pose call spent 36 us outside its
+// kernel: two copies, and a blocking copy of the status word after the wait.
+// Larger calls copy their results, and the status word with them.
+constexpr int HOST_WRITE_POSES = 4096;
+// the context's page-locked status word, cleared
+cudaError_t status_word(lkg_ctx* ctx, int** word);
+// after the wait: ok unless the launch flagged an error
+int check_status_seen(lkg_ctx* ctx, const int* word);
 int check_status_word(int* d_status);
 // status word of the no-allocation entry point's array on the context's device
 int noalloc_check_status(lkg_ctx* ctx);
@@ -202,7 +212,7 @@ size_t group_spill_bytes(lkg_ctx* ctx, const Group& g, bool exact);
 // launch one prepared group (kernel launches only: stream-capturable)
 int launch_group(lkg_ctx* ctx, const Group& g, const char* d_tables, Scratch& sc, const double* d_poses,
                  double* d_scores, double* d_parts, int raw_pairs, int solv_only, float* atom_e, float* atom_v,
-                 const unsigned char* pose_mask = nullptr, double* d_iface = nullptr);
+                 const unsigned char* pose_mask = nullptr, double* d_iface = nullptr, int* host_status = nullptr);
 // a plan's launch group(s) scoring only the poses whose mask byte is set
 int plan_launch_masked(lkg_plan* plan, const double* d_poses, double* d_scores, const unsigned char* d_mask);
 void field_geometry(const double* coords, int n, double lo[3], int dims[3], double* spacing);

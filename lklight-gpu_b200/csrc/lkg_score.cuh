@@ -546,8 +546,13 @@ __device__ __forceinline__ void write_pose(const LaunchParams& p, const ComplexD
 
 __device__ __forceinline__ void finish_launch(const LaunchParams& p) {
     if (threadIdx.x == 0) {
+        if (p.host_status) __threadfence();   // the block's error flags before it counts as done
         unsigned long long d = atomicAdd(p.work_counter + 1, 1ull);
-        if (d == gridDim.x - 1) { p.work_counter[0] = 0ull; p.work_counter[1] = 0ull; }
+        if (d == gridDim.x - 1) {
+            p.work_counter[0] = 0ull;
+            p.work_counter[1] = 0ull;
+            if (p.host_status) *reinterpret_cast<volatile int*>(p.host_status) = atomicAdd(p.status, 0);
+        }
     }
 }
 
