@@ -363,6 +363,36 @@ __device__ __noinline__ void w_band(const ComplexDev& c, const WSlots<G>& W, int
     }
 }
 
+// The first n (<= 32) waiting pairs with a tagged atom that can lie within
+// 3.9 A, one a lane: re-tested in f64 (the slot position as f32 value +
+// residual, ~2^-48 relative), which sets the pose's interface bits.
+template <int G, bool DESOLV>
+__device__ __forceinline__ void w_tags(const ComplexDev& c, const WSlots<G>& W, const WDes<G>* D, const unsigned* hit,
+                                       int lane, int set, int n) {
+    if (lane >= n || !W.iset) return;
+    const unsigned e = hit[lane];
+    const int l = (int)(e >> 26), k = (int)(e & 0x3ffffffu);
+    const double4 a64 = c.rpos64[k];
+    double ex, ey, ez;
+    if (DESOLV) {
+        ex = D->lx[set + l] - a64.x;
+        ey = D->ly[set + l] - a64.y;
+        ez = D->lz[set + l] - a64.z;
+    } else {
+        const WPair& P = W.pair[l >> 1];
+        const int h = l & 1;
+        ex = ((double)P.x[h] + (double)P.rx[h]) - a64.x;
+        ey = ((double)P.y[h] + (double)P.ry[h]) - a64.y;
+        ez = ((double)P.z[h] + (double)P.rz[h]) - a64.z;
+    }
+    if (ex * ex + ey * ey + ez * ez <= IFACE2_D) {
+        const int2 rt = __ldg(c.rtag + k);
+        iface_set(W.iset, rt.x);
+        iface_set(W.iset, rt.y);
+        iface_set(W.iset, W.ltag[l]);
+    }
+}
+
 // Scores n listed candidates (from list[first]) of quad `quad` densely: 16
 // candidates a step, lane = (candidate, slot pair), the slot pair in
 // registers, two steps side by side (two receptor atoms in flight, two
@@ -371,8 +401,8 @@ __device__ __noinline__ void w_band(const ComplexDev& c, const WSlots<G>& W, int
 // CLASH: the complex's terms.  The list is padded to a whole step.
 template <int G, bool DESOLV, bool IFACE, bool NP, bool ELEC, bool CLASH>
 __device__ __forceinline__ void w_dense(const ComplexDev& c, WSlots<G>& W, WDes<G>* D, MinHash64* hash, int* status,
-                                        unsigned* iset, int lane, int set, int quad, int first, int n, WAcc& acc,
-                                        float& off, int& nhit, int& old_hits) {
+                                        int lane, int set, int quad, int first, int n, WAcc& acc, float& off,
+                                        int& nhit, int& old_hits, unsigned* thit, int& ntag) {
     constexpr unsigned FULL = 0xffffffffu;
     const int half = lane & 1;
     const WPair P = W.pair[quad * 2 + half];
@@ -380,8 +410,8 @@ __device__ __forceinline__ void w_dense(const ComplexDev& c, WSlots<G>& W, WDes<
     const float4* rpk = c.rpk;
     const F2 one = f2(W.one[0], W.one[1]);
     const int slot0 = quad * 4 + half * 2;
-    // IFACE: a slot of the pair is tagged (untagged receptor atoms matter then)
-    const bool tagged = IFACE && iset && (W.ltag[slot0] >= 0 || W.ltag[slot0 + 1] >= 0);
+    // IFACE: the slot is tagged (untagged receptor atoms matter then)
+    const bool tag0 = IFACE && W.ltag[slot0] >= 0, tag1 = IFACE && W.ltag[slot0 + 1] >= 0;
     float lf0 = 0.f, lf1 = 0.f;
     bool need0 = false, need1 = false;   // DESOLV: the slot's own minimum is wanted
     if (DESOLV) {
@@ -421,33 +451,24 @@ __device__ __forceinline__ void w_dense(const ComplexDev& c, WSlots<G>& W, WDes<
         acc.vdw = (acc.vdw + (double)(in0 ? v0 : 0.f)) + (double)(in1 ? v1 : 0.f);
         if (NP) acc.np += (int)in0 + (int)in1;
         off = fminf(off, fminf(fabsf(t0), fabsf(t1)));
-        // tagged atoms carry the sign bit on their heavy flag (receptor) or a
-        // tag (slot): re-tested in f64 (the slot position as f32 value +
-        // residual, ~2^-48 relative), which sets the pose's interface bits
-        // (few atoms are tagged, so the tags are asked first: one pair in
-        // thirty is near enough, and then the whole warp would wait)
-        if (IFACE && ((__float_as_uint(A.p.z) >> 31) | (unsigned)tagged) && fminf(d20, d21) <= IFACE2_F) {
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                const int lt = W.ltag[slot0 + h];
-                if (!iset || (h ? d21 : d20) > IFACE2_F || (lt < 0 && !(__float_as_uint(A.p.z) >> 31))) continue;
-                const double4 a64 = c.rpos64[k];
-                double ex, ey, ez;
-                if (DESOLV) {
-                    ex = D->lx[set + slot0 + h] - a64.x;
-                    ey = D->ly[set + slot0 + h] - a64.y;
-                    ez = D->lz[set + slot0 + h] - a64.z;
-                } else {
-                    const WPair& S = W.pair[quad * 2 + half];
-                    ex = ((double)S.x[h] + (double)S.rx[h]) - a64.x;
-                    ey = ((double)S.y[h] + (double)S.ry[h]) - a64.y;
-                    ez = ((double)S.z[h] + (double)S.rz[h]) - a64.z;
-                }
-                if (ex * ex + ey * ey + ez * ez <= IFACE2_D) {
-                    const int2 rt = __ldg(c.rtag + k);
-                    iface_set(iset, rt.x);
-                    iface_set(iset, rt.y);
-                    iface_set(iset, lt);
+        // pairs near enough with a tagged atom (the receptor's sign on its
+        // heavy flag, or a tagged slot) wait for w_tags
+        if (IFACE) {
+            const bool rt = __float_as_uint(A.p.z) >> 31;
+            const bool g0 = (rt || tag0) && d20 <= IFACE2_F, g1 = (rt || tag1) && d21 <= IFACE2_F;
+            const unsigned b0 = __ballot_sync(FULL, g0), b1 = __ballot_sync(FULL, g1);
+            if (b0 | b1) {
+                const unsigned lt_mask = (1u << lane) - 1u;
+                const int n0 = __popc(b0);
+                const unsigned e = ((unsigned)slot0 << 26) | k;
+                if (g0) thit[ntag + __popc(b0 & lt_mask)] = e;
+                if (g1) thit[ntag + n0 + __popc(b1 & lt_mask)] = e + (1u << 26);
+                ntag += n0 + __popc(b1);
+                __syncwarp();
+                while (ntag >= 32) {   // the last 32 first: the rest stays at the front
+                    ntag -= 32;
+                    w_tags<G, DESOLV>(c, W, D, thit + ntag, lane, set, 32);
+                    __syncwarp();
                 }
             }
         }
@@ -529,7 +550,8 @@ __device__ __forceinline__ void w_dense_exact(const ComplexDev& c, const WSlots<
 template <int G, bool DESOLV, bool IFACE, bool NP, bool STAGE, bool EXACT, class GroupOf>
 __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes<G>* D, MinHash64* hash, int* status,
                                          int lane, int first, int end, int step, GroupOf group_of, WAcc& acc,
-                                         WStage* S = nullptr, WExact<G>* X = nullptr, bool far_sep = false) {
+                                         WStage* S = nullptr, WExact<G>* X = nullptr, bool far_sep = false,
+                                         unsigned* thit = nullptr) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int NQ = (G + 3) / 4;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -790,6 +812,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
             //    the group goes on (the end of a list first, so its rest stays
             //    at the front), all at its end
             float off = 1e30f;
+            int ntag = 0;   // IFACE: tagged pairs waiting
 #pragma unroll
             for (int s = 0; s < NQ; ++s) {
                 // the length to score, and padding past the list's end
@@ -808,7 +831,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
 #pragma unroll 1
                 for (int s = 0; s < NQ; ++s)
                     w_dense<G, DESOLV, IFACE, NP, decltype(elec)::value, decltype(clash)::value>(
-                        c, W, D, hash, status, iset, lane, set, s, W.first[s], W.cnt[s], gsum, off, nhit, old_hits);
+                        c, W, D, hash, status, lane, set, s, W.first[s], W.cnt[s], gsum, off, nhit, old_hits, thit, ntag);
             };
             using T = std::true_type;
             using F = std::false_type;
@@ -826,6 +849,10 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
                 gsum.elec += r.elec;
                 gsum.vdw += r.vdw;
                 if (NP) gsum.np += r.np;
+            }
+            if (IFACE) {
+                __syncwarp();
+                w_tags<G, DESOLV>(c, W, D, thit, lane, set, ntag);
             }
             }
             __syncwarp();
@@ -880,6 +907,9 @@ __global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCK
     WExact<G>* X = EXACT ? reinterpret_cast<WExact<G>*>(wk_smem + (WK_THREADS / 32) * (sizeof(WSlots<G>) + sizeof(ComplexDev))) +
                                (threadIdx.x >> 5)
                          : nullptr;
+    // IFACE: tagged pairs waiting for w_tags
+    __shared__ unsigned s_thit[IFACE && !EXACT ? WK_THREADS / 32 : 1][96];
+    unsigned* const thit = IFACE && !EXACT ? s_thit[threadIdx.x >> 5] : nullptr;
     if (STAGE) {
         if (lane == 0) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(w_smem_u32(&S->bar)), "r"(1));
@@ -931,7 +961,7 @@ __global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCK
         __syncwarp();
         WAcc acc;
         w_groups<G, false, IFACE, NP, STAGE, EXACT>(c, W, nullptr, nullptr, p.status, lane, g0, g1, 1,
-                                                    [](int k) { return k; }, acc, S, X);
+                                                    [](int k) { return k; }, acc, S, X, false, thit);
         if (IFACE && W.ibits) w_iface_flush(W, c);
         double* const pose_part = p.partials + 4 * first_part;
         if (!p.sub) {
@@ -1026,6 +1056,8 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
     __shared__ ComplexDev s_c;
     __shared__ unsigned s_near[WD_NEAR / 32];
     __shared__ unsigned short s_list[WD_NEAR];
+    __shared__ unsigned s_thit[IFACE ? NW : 1][96];
+    unsigned* const thit = IFACE ? s_thit[threadIdx.x >> 5] : nullptr;
     const int lane = w_lane(), wid = threadIdx.x >> 5;
     unsigned long long* const spill =
         p.spill ? reinterpret_cast<unsigned long long*>(p.spill + (size_t)blockIdx.x * p.spill_cap * SPILL_SLOT_BYTES)
@@ -1089,7 +1121,8 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
             __syncthreads();
             // warp k scores the near groups k, k + NW, ...
             w_groups<G, true, IFACE, NP, false, false>(c, W, D, &hash, p.status, lane, wid, total, NW,
-                                         [&](int k) { return g0 + s_list[k]; }, acc, nullptr, nullptr, far_sep);
+                                         [&](int k) { return g0 + s_list[k]; }, acc, nullptr, nullptr, far_sep,
+                                                       thit);
             if (g0 + WD_NEAR < ngrp) __syncthreads();   // the list is read
         }
         if (IFACE && W.ibits) w_iface_flush(W, c);   // before the block's barrier below
