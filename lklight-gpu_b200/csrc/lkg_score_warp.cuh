@@ -40,8 +40,12 @@ namespace lkg {
 constexpr int WK_THREADS = 128;   // 4 independent warps per block
 
 // candidates a quad's list holds: lists are scored when one holds more than
-// W_LIST - 64 (two chunks add at most 64)
-constexpr int W_LIST = 128;
+// W_LIST - 64 (two chunks add at most 64).  Long enough that most groups are
+// scored once, at their end, short enough to leave L1 its room.  ms at 96 / 128
+// / 192 / 256 / 384 / 512: 1800 vdw poses with groups of 8: 0.89 / 0.85 / 0.83
+// / 0.80 / 0.81 / 0.84; sixteen complexes with groups of 16: 13.0 / 12.1 / 11.9
+// / 12.0 / 12.5 / 15.6.
+template <int G> constexpr int W_LIST = G <= 8 ? 256 : 192;
 
 // resident blocks per SM the register budget is sized for: 72 registers (a
 // few spills in the cold parts).  Sixteen complexes of 2,000 poses: 12.5 ms at
@@ -83,7 +87,7 @@ struct WSlots {
     Rot rot;                          // pose of the current work unit
     WPair pair[G / 2];
     float4 quad[(G + 3) / 4];         // candidate test of each quad's sphere: -2 c', R^2 - |c'|^2 (c' = c - group centre)
-    unsigned list[(G + 3) / 4][W_LIST + 16];   // receptor indices of each quad's candidates (and padding)
+    unsigned list[(G + 3) / 4][W_LIST<G> + 16];   // receptor indices of each quad's candidates (and padding)
     int first[(G + 3) / 4], cnt[(G + 3) / 4];   // the part of each list that is scored
     float one[2];                     // 1, 1 (see w_d2)
     double* part;                     // the unit's group partials (split tiles), or null
@@ -699,7 +703,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
             int m = cnt[0];
 #pragma unroll
             for (int s = 1; s < NQ; ++s) m = max(m, cnt[s]);
-            return m > W_LIST - 64;
+            return m > W_LIST<G> - 64;
         };
         const float4 far_away = make_float4(3e30f, 3e30f, 3e30f, 0.f);
         int r0 = -32;                                     // the current 32 rows
