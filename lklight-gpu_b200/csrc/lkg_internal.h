@@ -90,6 +90,9 @@ struct ComplexDev {
 //   IF_VDW: s = s + pr*s + pl*s, no membrane    (vdw.rs:146-149)
 enum { IF_NONE = 0, IF_DNA = 1, IF_SUM = 2, IF_VDW = 3 };
 
+// poses a launch can carry in its own parameters
+constexpr int PARAM_POSES = 16;
+
 // One launch over a batch of (complex, pose range) items.
 struct LaunchParams {
     const ComplexDev* cx;        // device array of complex descriptors
@@ -107,6 +110,8 @@ struct LaunchParams {
     int tile;                    // ligand atoms per work unit (non-desolv kernel)
     int group;                   // ligand atoms per candidate-search group
     const double* poses;         // global N x 7 (w,x,y,z,tx,ty,tz)
+    int n_param;                 // > 0: the poses are param_poses instead (calls of a few host poses: no copy to wait for)
+    double param_poses[7 * PARAM_POSES];
     double* scores;              // [N] final score, or N x 2 raw (elec, vdw) when raw_pairs
     double* parts;               // [N x 4] or null: elec_raw, vdw, solv, near pairs
     int raw_pairs;               // compat: scores holds (elec_raw, vdw) pairs

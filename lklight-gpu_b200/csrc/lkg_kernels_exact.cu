@@ -30,7 +30,6 @@ cudaError_t launch_score_exact(const LaunchParams& p, int blocks, cudaStream_t s
     if (p.tile % p.group) return cudaErrorInvalidValue;
     switch (p.group) {
         case 4: return launch_exact_g<4>(p, blocks, s);
-        case 8: return launch_exact_g<8>(p, blocks, s);
         case 16: return launch_exact_g<16>(p, blocks, s);
         default: return launch_exact_g<32>(p, blocks, s);
     }
@@ -55,7 +54,6 @@ static int occ_exact_g() {
 int max_blocks_score_exact(int group) {
     switch (group) {
         case 4: return occ_exact_g<4>();
-        case 8: return occ_exact_g<8>();
         case 16: return occ_exact_g<16>();
         default: return occ_exact_g<32>();
     }

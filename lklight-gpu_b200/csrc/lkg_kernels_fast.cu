@@ -41,7 +41,6 @@ cudaError_t launch_score_fast(const LaunchParams& p, int threads, int blocks, cu
     if (p.tile % p.group) return cudaErrorInvalidValue;
     switch (p.group) {
         case 4: return launch_warp_g<4>(p, blocks, s);
-        case 8: return launch_warp_g<8>(p, blocks, s);
         case 16: return launch_warp_g<16>(p, blocks, s);
         default: return launch_warp_g<32>(p, blocks, s);
     }
@@ -86,7 +85,6 @@ cudaError_t launch_far_poses(const LaunchParams& p, int blocks, cudaStream_t s) 
 cudaError_t launch_desolv_fast(const LaunchParams& p, int threads, int blocks, int hcap, cudaStream_t s) {
     switch (p.group) {
         case 4: return launch_warp_desolv_g<4>(p, blocks, hcap, s);
-        case 8: return launch_warp_desolv_g<8>(p, blocks, hcap, s);
         case 16: return launch_warp_desolv_g<16>(p, blocks, hcap, s);
         default: break;
     }
@@ -111,7 +109,6 @@ static int occ_warp_desolv_g(int hcap) {
 int max_blocks_score_fast(int /*threads*/, int group) {
     switch (group) {
         case 4: return occ_warp_g<4>();
-        case 8: return occ_warp_g<8>();
         case 16: return occ_warp_g<16>();
         default: return occ_warp_g<32>();
     }
@@ -119,7 +116,6 @@ int max_blocks_score_fast(int /*threads*/, int group) {
 int max_blocks_desolv_fast(int threads, int hcap, int group) {
     switch (group) {
         case 4: return occ_warp_desolv_g<4>(hcap);
-        case 8: return occ_warp_desolv_g<8>(hcap);
         case 16: return occ_warp_desolv_g<16>(hcap);
         default: break;
     }

@@ -324,16 +324,17 @@ void bisect_groups(const double* c, int* idx, int n, int G) {
     bisect_groups(c, idx + left, n - left, G);
 }
 
-// ligand: bisection order in groups of ctx->group atoms
+// ligand: bisection order in the groups that are searched together
 int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
     ComplexDev& d = cr.d;
     const int n = L.n;
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
-    bisect_groups(L.c.data(), order.data(), n, ctx->group);
-    const std::vector<int> coarse = order;
-    for (int k = 0; k < n; k += ctx->group)   // and quads compact inside each group
-        bisect_groups(L.c.data(), order.data() + k, std::min(ctx->group, n - k), 4);
+    std::vector<int> coarse = order;   // in groups of ctx->group (the surrogate's anchors)
+    bisect_groups(L.c.data(), coarse.data(), n, ctx->group);
+    bisect_groups(L.c.data(), order.data(), n, ctx->scan());
+    for (int k = 0; k < n; k += ctx->scan())   // and quads compact inside each group
+        bisect_groups(L.c.data(), order.data() + k, std::min(ctx->scan(), n - k), 4);
     std::vector<int> at(n);
     for (int k = 0; k < n; ++k) at[order[k]] = k;
     cr.lgroup_order.resize(n);
@@ -351,9 +352,9 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
         par64[k] = make_double4(L.svdw[i], L.rad[i], L.eps[i], L.heavy[i] ? 1.0 : 0.0);
         sol64[k] = make_double2(L.des[i], L.asa[i]);
     }
-    // bounding spheres (ligand frame) of every group of ctx->group and every
+    // bounding spheres (ligand frame) of every searched group and every
     // quad of 4 consecutive atoms, for the warp kernels' candidate search
-    const int G = ctx->group;
+    const int G = ctx->scan();
     auto spheres = [&](int step) {
         std::vector<float4> out(std::max((n + step - 1) / step, 1));
         for (int gi = 0; gi * step < n; ++gi) {
@@ -451,8 +452,8 @@ int occupancy(lkg_ctx* ctx, bool desolv, bool exact, int threads, int hcap) {
     Occupancy& o = desolv ? ctx->occ_desolv[exact] : ctx->occ_tiles[exact];
     if (o.threads == threads && o.hcap == hcap && o.blocks > 0) return o.blocks;
     int b;
-    if (desolv) b = exact ? max_blocks_desolv_exact(threads, hcap) : max_blocks_desolv_fast(threads, hcap, ctx->group);
-    else b = exact ? max_blocks_score_exact(ctx->group) : max_blocks_score_fast(threads, ctx->group);
+    if (desolv) b = exact ? max_blocks_desolv_exact(threads, hcap) : max_blocks_desolv_fast(threads, hcap, ctx->scan());
+    else b = exact ? max_blocks_score_exact(ctx->scan()) : max_blocks_score_fast(threads, ctx->scan());
     o.threads = threads; o.hcap = hcap; o.blocks = std::max(1, b);
     return o.blocks;
 }
@@ -650,20 +651,20 @@ static void split_tiles(lkg_ctx* ctx, Group& G) {
     if (G.ic.empty()) return;
     const long long want = SPLIT_UNITS * (long long)ctx->sm_count * occupancy(ctx, false, false, ctx->tile, 0) *
                            (128 / 32);
-    int sub = ctx->tile / ctx->group;
+    int sub = ctx->tile / ctx->scan();
     auto units = [&](int s) {
         long long n = 0;
         for (size_t i = 0; i < G.ic.size(); ++i) {
-            const long long ng = (ctx->cx[G.ic[i]]->d.nl + ctx->group - 1) / ctx->group;
+            const long long ng = (ctx->cx[G.ic[i]]->d.nl + ctx->scan() - 1) / ctx->scan();
             n += G.inp[i] * ((ng + s - 1) / s);
         }
         return n;
     };
     while (sub > 1 && units(sub) < want) sub >>= 1;
-    if (sub == ctx->tile / ctx->group) return;
+    if (sub == ctx->tile / ctx->scan()) return;
     G.sub = sub;
     for (size_t i = 0; i < G.ic.size(); ++i) {
-        const long long ng = (ctx->cx[G.ic[i]]->d.nl + ctx->group - 1) / ctx->group;
+        const long long ng = (ctx->cx[G.ic[i]]->d.nl + ctx->scan() - 1) / ctx->scan();
         G.ws.push_back(G.ws.back() + G.inp[i] * ((ng + sub - 1) / sub));
         G.g0.push_back(G.g0.back() + G.inp[i] * ng);
     }
@@ -719,7 +720,7 @@ size_t group_spill_bytes(lkg_ctx* ctx, const Group& G, bool exact) {
 
 int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, const double* d_poses,
                  double* d_scores, double* d_parts, int raw_pairs, int solv_only, float* atom_e, float* atom_v,
-                 const unsigned char* pose_mask, double* d_iface, int* host_status) {
+                 const unsigned char* pose_mask, double* d_iface, int* host_status, const double* h_poses, int n_host) {
     const bool exact = ctx->precision == LKG_PREC_EXACT;
     const int ni = (int)G.ic.size();
     LaunchParams p{};
@@ -734,8 +735,12 @@ int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, cons
     p.n_items = ni;
     p.total_work = split ? G.ws.back() : G.w0.back();
     p.tile = ctx->tile;
-    p.group = ctx->group;
+    p.group = ctx->scan();
     p.poses = d_poses;
+    if (h_poses) {
+        p.n_param = n_host;
+        memcpy(p.param_poses, h_poses, (size_t)n_host * 7 * sizeof(double));
+    }
     p.scores = d_scores;
     p.parts = d_parts;
     p.raw_pairs = raw_pairs;
@@ -799,7 +804,7 @@ int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, cons
 
 int launch_items(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, const double* d_poses,
                  double* d_scores, double* d_parts, int raw_pairs, int solv_only, float* atom_e,
-                 float* atom_v, double* d_iface, int* host_status) {
+                 float* atom_v, double* d_iface, int* host_status, const double* h_poses) {
     if (n_items <= 0) return set_ok();
     Group g[2];
     size_t n_poses = 0;
@@ -826,7 +831,7 @@ int launch_items(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, c
     for (int k = 0; k < 2; ++k) {
         if (g[k].ic.empty()) continue;
         st = launch_group(ctx, g[k], ctx->d_items.as<char>() + (k ? b0 : 0), ctx->scratch, d_poses, d_scores, d_parts,
-                          raw_pairs, solv_only, atom_e, atom_v, nullptr, d_iface, host_status);
+                          raw_pairs, solv_only, atom_e, atom_v, nullptr, d_iface, host_status, h_poses, (int)n_poses);
         if (st) return st;
     }
     return set_ok();
@@ -1093,13 +1098,16 @@ static int score_host(lkg_ctx* ctx, int id, int n, const double* poses, double* 
     cudaSetDevice(ctx->device);
     const size_t pb = (size_t)n * 7 * sizeof(double), ob = (size_t)n * sizeof(double),
                  qb = (size_t)n * 4 * sizeof(double), ib = (size_t)n * 3 * sizeof(double);
-    LKG_CK(ctx->h_poses.reserve(pb), "staging");
+    const bool in_launch = n <= PARAM_POSES;
     LKG_CK(ctx->h_out.reserve(ob + qb + ib), "staging");
-    LKG_CK(ctx->d_poses.reserve(pb), "staging");
     int* status = nullptr;
     LKG_CK(status_word(ctx, &status), "staging");
-    memcpy(ctx->h_poses.p, poses, pb);
-    LKG_CK(cudaMemcpyAsync(ctx->d_poses.p, ctx->h_poses.p, pb, cudaMemcpyHostToDevice, ctx->stream), "pose upload");
+    if (!in_launch) {
+        LKG_CK(ctx->h_poses.reserve(pb), "staging");
+        LKG_CK(ctx->d_poses.reserve(pb), "staging");
+        memcpy(ctx->h_poses.p, poses, pb);
+        LKG_CK(cudaMemcpyAsync(ctx->d_poses.p, ctx->h_poses.p, pb, cudaMemcpyHostToDevice, ctx->stream), "pose upload");
+    }
     int st;
     if (n <= HOST_WRITE_POSES) {
         double* h_scores = ctx->h_out.as<double>();
@@ -1107,7 +1115,7 @@ static int score_host(lkg_ctx* ctx, int id, int n, const double* poses, double* 
         double* h_iface = (double*)(ctx->h_out.as<char>() + ob + qb);
         if (iface) memset(h_iface, 0, ib);   // zeros for a complex without restraints
         if ((st = launch_items(ctx, 1, &id, &n, ctx->d_poses.as<double>(), h_scores, parts ? h_parts : nullptr, 0, 0,
-                               nullptr, nullptr, iface ? h_iface : nullptr, status)))
+                               nullptr, nullptr, iface ? h_iface : nullptr, status, in_launch ? poses : nullptr)))
             return st;
         if ((st = wait_stream(ctx, 300.0))) return st;
         if ((st = check_status_seen(ctx, status))) return st;

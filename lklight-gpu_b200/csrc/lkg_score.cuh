@@ -49,6 +49,11 @@ template <> struct Tr<double> {
 // ------------------------------------------------------------------------
 // transform
 // ------------------------------------------------------------------------
+// pose g of the launch
+__device__ __forceinline__ const double* pose_of(const LaunchParams& p, long long g) {
+    return p.n_param ? p.param_poses + 7 * g : p.poses + 7 * g;
+}
+
 struct Rot { double m00, m01, m02, m10, m11, m12, m20, m21, m22, tx, ty, tz; };
 
 __device__ __forceinline__ Rot pose_matrix(const double* __restrict__ pq) {
@@ -560,7 +565,7 @@ __device__ __forceinline__ void finish_launch(const LaunchParams& p) {
 // kernel 1: tiles of ligand atoms (dna / pydock / vdw and compat flags)
 // ------------------------------------------------------------------------
 template <typename R>
-__global__ void __launch_bounds__(256) k_score_tiles(LaunchParams p) {
+__global__ void __launch_bounds__(256) k_score_tiles(const __grid_constant__ LaunchParams p) {
     __shared__ long long s_work;
     __shared__ double s_red[4][32];
     for (;;) {
@@ -579,7 +584,7 @@ __global__ void __launch_bounds__(256) k_score_tiles(LaunchParams p) {
         AtomAcc acc{0.0, 0.0, 0};
         unsigned* ibits = iface_bits(p, c, g);
         if (j < c.nl && threadIdx.x < p.tile) {
-            const Rot rot = pose_matrix(p.poses + 7 * g);
+            const Rot rot = pose_matrix(pose_of(p, g));
             double dummy_min = 0.0;
             const bool atom_out = p.atom_elec && b == 0 && pose == 0;
             Atom<R>::template run<false>(c, rot, j, acc, dummy_min, nullptr, p.status,
@@ -613,7 +618,7 @@ __global__ void __launch_bounds__(256) k_score_tiles(LaunchParams p) {
 // kernel 2: one block per pose, cpydock desolvation fused
 // ------------------------------------------------------------------------
 template <typename R>
-__global__ void __launch_bounds__(512) k_score_desolv(LaunchParams p) {
+__global__ void __launch_bounds__(512) k_score_desolv(const __grid_constant__ LaunchParams p) {
     extern __shared__ __align__(16) char smem[];
     __shared__ long long s_work;
     __shared__ double s_red[4][32];
@@ -634,7 +639,7 @@ __global__ void __launch_bounds__(512) k_score_desolv(LaunchParams p) {
         MinHash hash;
         hash.init(smem, c.hcap, spill, p.spill_cap, &s_spilled);
         __syncthreads();
-        const Rot rot = pose_matrix(p.poses + 7 * g);
+        const Rot rot = pose_matrix(pose_of(p, g));
         unsigned* ibits = iface_bits(p, c, g);
         AtomAcc acc{0.0, 0.0, 0};
         double solv_l = 0.0;

@@ -896,7 +896,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
 // NP: near pairs are counted (launches with parts)
 // EXACT: f64 pair math in the reference's operation order
 template <int G, bool IFACE, bool NP, bool STAGE = false, bool EXACT = false>
-__global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCKS) k_score_warp(LaunchParams p) {
+__global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCKS) k_score_warp(const __grid_constant__ LaunchParams p) {
     static_assert(G == 4 || G == 8 || G == 16 || G == 32, "group size");
     static_assert(!(STAGE && (IFACE || EXACT)), "the staged variant is the plain kernel's");
     constexpr unsigned FULL = 0xffffffffu;
@@ -926,10 +926,17 @@ __global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCK
     if (lane < 2) W.one[lane] = p.one;
     __syncwarp();
     int cur = -1;   // complex whose descriptor c holds
-    for (;;) {
-        unsigned long long wq = 0;
-        if (lane == 0) wq = atomicAdd(p.work_counter, 1ull);
-        const long long w = (long long)__shfl_sync(FULL, wq, 0);
+    // the first unit of every warp is fixed (spread over the blocks first), the
+    // others come from the counter
+    const long long nwarps = (long long)gridDim.x * (WK_THREADS / 32);
+    for (bool first = true;; first = false) {
+        long long w = (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+        if (!first) {
+            if (p.total_work <= nwarps) break;
+            unsigned long long wq = 0;
+            if (lane == 0) wq = atomicAdd(p.work_counter, 1ull);
+            w = nwarps + (long long)__shfl_sync(FULL, wq, 0);
+        }
         if (w >= p.total_work) break;
         const int b = find_item(p.item_work0, p.n_items, w);
         const int cid = __ldg(p.item_complex + b);
@@ -951,7 +958,7 @@ __global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCK
         if (p.pose_mask && !p.pose_mask[g]) continue;   // pose skipped: keeps its score
         __syncwarp();   // readers of the previous unit's pose are done
         if (lane == 0) {
-            W.rot = pose_matrix(p.poses + 7 * g);
+            W.rot = pose_matrix(pose_of(p, g));
             if (IFACE) w_iface_begin(W, c, iface_bits(p, c, g));
             else if (c.iface_words) atomicOr(p.status, 2);   // a launch without room for the bits
         }
@@ -1050,7 +1057,7 @@ __host__ __device__ constexpr size_t wd_smem(int hcap) {
 }
 
 template <int G, bool IFACE, bool NP>
-__global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(LaunchParams p) {
+__global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(const __grid_constant__ LaunchParams p) {
     constexpr int NW = WD_THREADS / 32;
     extern __shared__ __align__(16) unsigned char wd_smem_raw[];
     __shared__ long long s_work;
@@ -1088,7 +1095,7 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
         if (lane < 2) W.one[lane] = p.one;
         if (IFACE) W.ibuf[lane] = 0u;   // the slots move with the complex's hash size
         if (lane == 0) {
-            W.rot = pose_matrix(p.poses + 7 * g);
+            W.rot = pose_matrix(pose_of(p, g));
             if (IFACE) w_iface_begin(W, c, iface_bits(p, c, g));
             else if (c.iface_words) atomicOr(p.status, 2);
         }
@@ -1174,7 +1181,7 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(Lau
 // per SM resident; here every thread has independent gathers in flight.
 // Skipped (masked) poses are left alone.
 constexpr int FAR_THREADS = 256;
-static __global__ void __launch_bounds__(FAR_THREADS, 4) k_far_poses(LaunchParams p) {
+static __global__ void __launch_bounds__(FAR_THREADS, 4) k_far_poses(const __grid_constant__ LaunchParams p) {
     __shared__ double s_red[4][32];
     for (long long w = blockIdx.x; w < p.total_work; w += gridDim.x) {
         const int b = find_item(p.item_work0, p.n_items, w);
@@ -1183,7 +1190,7 @@ static __global__ void __launch_bounds__(FAR_THREADS, 4) k_far_poses(LaunchParam
         if (p.pose_mask && !p.pose_mask[g]) continue;   // block-uniform
         double v[1] = {0.0};
         if (c.flags & F_FAR) {
-            const Rot rot = pose_matrix(p.poses + 7 * g);
+            const Rot rot = pose_matrix(pose_of(p, g));
             for (int j = threadIdx.x; j < c.nl; j += FAR_THREADS) {
                 if (__ldg(&c.lpos[j].w) == 0.f) continue;
                 const double4 b64 = c.lpos64[j];
