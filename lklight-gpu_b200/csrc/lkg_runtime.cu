@@ -641,9 +641,9 @@ void Group::pack(char* dst) const {
 // tiles, halved until there are as many, down to one group of atoms.  A warp
 // works through a unit's groups one after another, each a chain of dependent
 // loads of several us, so one pose took as long as a tile's 8-16 groups
-// (config-0 sizes: 194 us, now 63), and the warps that a small launch left
+// (config-0 sizes: 170 us, 62 when split), and the warps that a small launch left
 // idle waited for the others (301 poses of a protein-density complex: 715 us,
-// now 308).  2, 8 and 1000 units a slot measured alike, but each group's
+// then 308).  2, 8 and 1000 units a slot measured alike, but each group's
 // partial is 32 bytes to allocate (1 ms more on the first call with 1800 poses
 // at 8).  The score's bits are the same either way.
 constexpr int SPLIT_UNITS = 2;
