@@ -280,7 +280,7 @@ int cuda_far_field(const float* phi, int nx, int ny, int nz, float ox, float oy,
         if (C.fields.size() >= 8) C.fields.clear();
         fb = std::make_shared<DBuf>();
         if ((e = fb->reserve(np * sizeof(float))) == cudaSuccess)
-            e = cudaMemcpy(fb->p, phi, np * sizeof(float), cudaMemcpyHostToDevice);
+            e = to_device(fb->p, phi, np * sizeof(float), ctx->stream);
         if (e != cudaSuccess) {
             set_error(cuda_to_status(e), "field upload: %s", cudaGetErrorString(e));
             return report("cuda_far_field", cuda_to_status(e), 1, n);

@@ -1345,16 +1345,19 @@ int lkg_surrogate_create(lkg_ctx* ctx, int complex_id, uint64_t seed, lkg_surrog
             return set_error(cuda_to_status(e), "surrogate alloc: %s", cudaGetErrorString(e));
         }
     }
-    cudaMemcpy(S->p.p, p.data(), NPARAM * 4, cudaMemcpyHostToDevice);
-    cudaMemset(S->m1.p, 0, NPARAM * 4);
-    cudaMemset(S->m2.p, 0, NPARAM * 4);
+    cudaStream_t s = ctx->stream;
+    if ((e = to_device(S->p.p, p.data(), NPARAM * 4, s)) != cudaSuccess ||
+        (e = cudaMemsetAsync(S->m1.p, 0, NPARAM * 4, s)) != cudaSuccess ||
+        (e = cudaMemsetAsync(S->m2.p, 0, NPARAM * 4, s)) != cudaSuccess ||
+        (e = cudaMemsetAsync(S->d_status.p, 0, sizeof(int), s)) != cudaSuccess ||
+        (e = to_device(S->anchors.p, anc.data(), NA * sizeof(int), s)) != cudaSuccess) {
+        delete S;
+        return set_error(cuda_to_status(e), "surrogate init: %s", cudaGetErrorString(e));
+    }
     const int one = 1;
     const int step0[2] = {one, 0};   // t = 1, no block done
-    cudaMemcpy(S->d_step.p, step0, sizeof(step0), cudaMemcpyHostToDevice);
-    cudaMemset(S->d_status.p, 0, sizeof(int));
-    cudaMemcpy(S->anchors.p, anc.data(), NA * sizeof(int), cudaMemcpyHostToDevice);
     if ((rc = refresh_bf16(S))) { delete S; return rc; }
-    if ((e = cudaDeviceSynchronize()) != cudaSuccess) {
+    if ((e = to_device(S->d_step.p, step0, sizeof(step0), s)) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) {
         delete S;
         return set_error(cuda_to_status(e), "surrogate init: %s", cudaGetErrorString(e));
     }
@@ -1502,7 +1505,7 @@ int lkg_surrogate_status(lkg_surrogate* S, int* bits) {
     cudaSetDevice(S->ctx->device);
     LKG_CK(cudaStreamSynchronize(S->ctx->stream), "surrogate status");
     LKG_CK(cudaMemcpy(bits, S->d_status.p, sizeof(int), cudaMemcpyDeviceToHost), "surrogate status");
-    LKG_CK(cudaMemset(S->d_status.p, 0, sizeof(int)), "surrogate status");
+    LKG_CK(cudaMemsetAsync(S->d_status.p, 0, sizeof(int), S->ctx->stream), "surrogate status");
     return set_ok();
 }
 
@@ -1515,7 +1518,7 @@ int lkg_surrogate_get_params(lkg_surrogate* S, float* out) {
 }
 int lkg_surrogate_set_params(lkg_surrogate* S, const float* in) {
     if (!S || !in) return set_error(LKG_ERR_ARG, "bad args");
-    LKG_CK(cudaMemcpy(S->p.p, in, NPARAM * 4, cudaMemcpyHostToDevice), "set params");
+    LKG_CK(to_device(S->p.p, in, NPARAM * 4, S->ctx->stream), "set params");
     int st = refresh_bf16(S);
     if (st) return st;
     LKG_CK(cudaStreamSynchronize(S->ctx->stream), "set params");
@@ -1530,8 +1533,8 @@ int lkg_surrogate_grad(lkg_surrogate* S, int n, const uint16_t* feats, const flo
     if (!S || n <= 0 || !feats || !targets) return set_error(LKG_ERR_ARG, "bad grad args");
     cudaSetDevice(S->ctx->device);
     if (sur_reserve(S, n, true)) return lkg_last_status();
-    LKG_CK(cudaMemcpy(S->X.p, feats, (size_t)n * IN * 2, cudaMemcpyHostToDevice), "grad upload");
-    LKG_CK(cudaMemcpy(S->t.p, targets, (size_t)n * 4, cudaMemcpyHostToDevice), "grad upload");
+    LKG_CK(to_device(S->X.p, feats, (size_t)n * IN * 2, S->ctx->stream), "grad upload");
+    LKG_CK(to_device(S->t.p, targets, (size_t)n * 4, S->ctx->stream), "grad upload");
     LKG_CK(cudaMemsetAsync(S->loss.p, 0, sizeof(float), S->ctx->stream), "grad loss clear");
     S->pdl = false;
     int st;

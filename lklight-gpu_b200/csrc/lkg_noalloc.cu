@@ -78,7 +78,7 @@ int noalloc_check_status(lkg_ctx* ctx) {
         if (ctx->device >= 0 && ctx->device < 64) base = g_addr[ctx->device];
     }
     if (!base) return set_ok();
-    return check_status_word(reinterpret_cast<int*>(static_cast<char*>(base) + OFF_STATUS));
+    return check_status_word(reinterpret_cast<int*>(static_cast<char*>(base) + OFF_STATUS), ctx->stream);
 }
 }  // namespace lkg
 

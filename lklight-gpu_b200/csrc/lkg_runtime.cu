@@ -492,7 +492,7 @@ static int set_rpar_tag_signs(lkg_ctx* ctx, ComplexRec& cr, const std::vector<in
         const bool tagged = rt && ((*rt)[k].x >= 0 || (*rt)[k].y >= 0);
         par[k].z = tagged ? -std::fabs(par[k].z) : std::fabs(par[k].z);
     }
-    LKG_CK(cudaMemcpy(cr.rpar.p, par.data(), nr * sizeof(float4), cudaMemcpyHostToDevice), "receptor tags");
+    LKG_CK(to_device(cr.rpar.p, par.data(), nr * sizeof(float4), ctx->stream), "receptor tags");
     return interleave_receptor(ctx, cr, nr);
 }
 
@@ -853,26 +853,31 @@ int wait_stream(lkg_ctx* ctx, double timeout_s) {
     }
 }
 
-int check_status_word(int* d_status) {
+static cudaError_t clear_status(int* d_status, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(d_status, 0, 4 * sizeof(int), s);
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
+int check_status_word(int* d_status, cudaStream_t s) {
     if (!d_status) return set_ok();
     int h[4] = {0, 0, 0, 0};
     LKG_CK(cudaMemcpy(h, d_status, sizeof(h), cudaMemcpyDeviceToHost), "status read");
     if (h[0] & 1) {
-        cudaMemset(d_status, 0, sizeof(h));
+        clear_status(d_status, s);
         return set_error(LKG_ERR_CAPACITY, "desolvation hash overflow (too many receptor atoms within 6.4 A of one pose)");
     }
     if (h[0] & 2) {
-        cudaMemset(d_status, 0, sizeof(h));
+        clear_status(d_status, s);
         return set_error(LKG_ERR_STATE, "restraints or membrane set after the batch was prepared: prepare it again");
     }
     if (h[0] & 8) {
-        cudaMemset(d_status, 0, sizeof(h));
+        clear_status(d_status, s);
         return set_error(LKG_ERR_TIMEOUT, "a staged candidate copy did not complete in time");
     }
     return set_ok();
 }
 
-int check_status(lkg_ctx* ctx) { return check_status_word(ctx->scratch.status.as<int>()); }
+int check_status(lkg_ctx* ctx) { return check_status_word(ctx->scratch.status.as<int>(), ctx->stream); }
 
 cudaError_t status_word(lkg_ctx* ctx, int** word) {
     const cudaError_t e = ctx->h_status.reserve(64);
@@ -1273,7 +1278,7 @@ int lkg_plan_create(lkg_ctx* ctx, int n_items, const int* ids, const int* counts
     P->b0 = b0;
     cudaError_t e;
     if ((e = P->d_tables.reserve(b0 + b1)) != cudaSuccess ||
-        (e = cudaMemcpy(P->d_tables.p, packed.data(), b0 + b1, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = to_device(P->d_tables.p, packed.data(), b0 + b1, ctx->stream)) != cudaSuccess ||
         (e = P->scratch.ensure(std::max<size_t>(P->g[0].partials(), 1), std::max<size_t>(P->n_poses, 1), ctx->stream,
                                P->n_poses * (size_t)P->g[0].iface_words)) != cudaSuccess ||
         (e = P->scratch.ensure_spill(std::max(group_spill_bytes(ctx, P->g[1], false),
@@ -1380,7 +1385,7 @@ int lkg_plan_sync(lkg_plan* P) {
     cudaSetDevice(P->ctx->device);
     int st = wait_stream(P->ctx, 300.0);
     if (st) return st;
-    return check_status_word(P->scratch.status.as<int>());
+    return check_status_word(P->scratch.status.as<int>(), P->ctx->stream);
 }
 
 }  // extern "C"

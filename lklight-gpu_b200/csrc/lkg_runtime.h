@@ -108,6 +108,15 @@ struct Scratch {
     cudaError_t ensure_spill(size_t bytes, cudaStream_t s);
 };
 
+// Host memory to the device in the order of stream s, complete on return.  A
+// plain cudaMemcpy from pageable memory may return while its last piece is on
+// its way, and the contexts' streams, created non-blocking, do not wait for it
+// (nor for a cudaMemset): their next kernel could read the old contents.
+inline cudaError_t to_device(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
 // one launch group's item tables: (complex, first pose, pose count) per item
 // and cumulative work units; `kind` 0 = tile kernels, 1 = fused desolvation.
 // sub > 0: the fast warp kernel takes units of `sub` ligand groups instead of
@@ -207,7 +216,7 @@ constexpr int HOST_WRITE_POSES = 4096;
 cudaError_t status_word(lkg_ctx* ctx, int** word);
 // after the wait: ok unless the launch flagged an error
 int check_status_seen(lkg_ctx* ctx, const int* word);
-int check_status_word(int* d_status);
+int check_status_word(int* d_status, cudaStream_t s);
 // status word of the no-allocation entry point's array on the context's device
 int noalloc_check_status(lkg_ctx* ctx);
 // item tables of the two launch groups for a batch
