@@ -353,7 +353,8 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
         sol64[k] = make_double2(L.des[i], L.asa[i]);
     }
     // bounding spheres (ligand frame) of every searched group and every
-    // quad of 4 consecutive atoms, for the warp kernels' candidate search
+    // quad of 4 consecutive atoms, for the warp kernels' candidate search;
+    // around the f32 centres that the kernels see
     const int G = ctx->scan();
     auto spheres = [&](int step) {
         std::vector<float4> out(std::max((n + step - 1) / step, 1));
@@ -362,7 +363,7 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
             double cen[3] = {0, 0, 0};
             for (int k = a0; k < a1; ++k)
                 for (int a = 0; a < 3; ++a) cen[a] += L.c[3 * order[k] + a];
-            for (int a = 0; a < 3; ++a) cen[a] /= (a1 - a0);
+            for (int a = 0; a < 3; ++a) cen[a] = (float)(cen[a] / (a1 - a0));
             double r2 = 0;
             for (int k = a0; k < a1; ++k) {
                 double dd = 0;
@@ -373,7 +374,27 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
         }
         return out;
     };
-    const std::vector<float4> grp = spheres(G), quad = spheres(4);
+    const std::vector<float4> grp = spheres(G);
+    std::vector<float4> quad = spheres(4);
+    // A quad's test, |a'|^2 - 2 a'.c' <= r^2 - |c'|^2 in f32 relative to the
+    // group's centre (r = SCAN_R + radius), is off by at most 18 roundings
+    // (2^-24) of M^2, M = |c'| + r, and a' and c' by 3 of M: both grow with the
+    // group's width, so the radius takes them (32 of |c'|^2 + r^2 and 8 of M;
+    // 1e-4 A in a compact group)
+    for (int k = 0; 4 * k < n; ++k) {
+        const float4 s = grp[4 * k / G];
+        float4& t = quad[k];
+        const double dx = (double)t.x - s.x, dy = (double)t.y - s.y, dz = (double)t.z - s.z;
+        const double cc = dx * dx + dy * dy + dz * dz, r = SCAN_R + t.w, g = r + 0x1p-21 * (std::sqrt(cc) + r);
+        t.w = (float)((std::sqrt(g * g + 0x1p-18 * (cc + g * g)) - SCAN_R) * (1.0 + 1e-7));
+    }
+    double ext2 = 0.0;
+    for (int k = 0; k < n; ++k) {
+        double dd = 0.0;
+        for (int a = 0; a < 3; ++a) dd += L.c[3 * k + a] * L.c[3 * k + a];
+        ext2 = std::max(ext2, dd);
+    }
+    d.lext = (float)(std::sqrt(3.0 * ext2) * (1.0 + 1e-6));
     cudaStream_t s = ctx->stream;
     LKG_CK(upload(cr.lgrp, grp, s), "upload ligand");
     LKG_CK(upload(cr.lquad, quad, s), "upload ligand");

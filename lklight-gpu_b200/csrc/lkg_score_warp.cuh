@@ -85,6 +85,7 @@ struct __align__(16) WPair {
 template <int G>
 struct WSlots {
     Rot rot;                          // pose of the current work unit
+    float scan;                       // and its search radius around an atom (w_pose)
     WPair pair[G / 2];
     float4 quad[(G + 3) / 4];         // candidate test of each quad's sphere: -2 c', R^2 - |c'|^2 (c' = c - group centre)
     unsigned list[(G + 3) / 4][W_LIST<G> + 16];   // receptor indices of each quad's candidates (and padding)
@@ -272,6 +273,18 @@ __device__ __forceinline__ int w_lane() {
     unsigned l;
     asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));
     return (int)l;
+}
+
+// The unit's pose, and the search radius of its atoms: SCAN_R grown by what f32
+// takes from the positions.  The receptor's and the centres' are rounded (2^-24
+// of a coordinate each), as are the distances to the cell rows (under 12
+// roundings of a coordinate; 2^-21 is 8 on the radius, 16 on its square).  1e-4 A
+// at 200 A, and at most 1 A, so that a pose at infinity does not search the whole
+// receptor: enough for coordinates up to 7e5 A.
+template <int G>
+__device__ __forceinline__ void w_pose(WSlots<G>& W, const ComplexDev& c, const double* pq) {
+    W.rot = pose_matrix(pq);
+    W.scan = SCAN_R + fminf(0x1p-21f * ((float)(fabs(pq[4]) + fabs(pq[5]) + fabs(pq[6])) + c.lext), 1.f);
 }
 
 // the descriptor of a unit's complex into shared memory by n threads (its
@@ -608,7 +621,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
                 if (lane >= Q0 && lane <= Q0 + NQ) {
                     const float4 s = lane == Q0 + NQ ? __ldg(c.lgrp + grp) : (quad ? __ldg(c.lquad + qi) : make_float4(0.f, 0.f, 0.f, 0.f));
                     b = make_double4((double)s.x, (double)s.y, (double)s.z, 0.0);
-                    rad = SCAN_R + s.w;
+                    rad = W.scan + s.w;
                 }
             };
             if (atom) b = c.lpos64[j];
@@ -664,9 +677,9 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
             gz = __shfl_sync(FULL, z, Q0 + NQ);
             R = __shfl_sync(FULL, rad, Q0 + NQ);
             if (lane >= Q0 && lane < Q0 + NQ) {
-                // |a' - c'|^2 <= R^2 as |a'|^2 - 2 a'.c' <= R^2 - |c'|^2 in the
-                // group frame (|a'| <= ~20 A: rounding ~1e-4, far inside the
-                // 0.02 A^2 that SCAN_R leaves); a quad past the ligand never passes
+                // |a' - c'|^2 <= r^2 as |a'|^2 - 2 a'.c' <= r^2 - |c'|^2 in the
+                // group frame (the rounding is in the quad's radius); a quad
+                // past the ligand never passes
                 const float lx = (float)(xd - (double)gx), ly = (float)(yd - (double)gy), lz = (float)(zd - (double)gz);
                 W.quad[lane - Q0] = quad ? make_float4(-2.f * lx, -2.f * ly, -2.f * lz,
                                                        rad * rad - (lx * lx + ly * ly + lz * lz))
@@ -958,7 +971,7 @@ __global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCK
         if (p.pose_mask && !p.pose_mask[g]) continue;   // pose skipped: keeps its score
         __syncwarp();   // readers of the previous unit's pose are done
         if (lane == 0) {
-            W.rot = pose_matrix(pose_of(p, g));
+            w_pose(W, c, pose_of(p, g));
             if (IFACE) w_iface_begin(W, c, iface_bits(p, c, g));
             else if (c.iface_words) atomicOr(p.status, 2);   // a launch without room for the bits
         }
@@ -1041,10 +1054,10 @@ constexpr int WD_BLOCKS = 3;
 constexpr int WD_NEAR = 1024;
 
 // whether a receptor atom can lie within reach of group gi (its sphere grown by
-// SCAN_R), by the receptor's distance bound at the posed centre
-__device__ __forceinline__ bool w_near(const ComplexDev& c, const Rot& rot, int gi) {
+// `scan`), by the receptor's distance bound at the posed centre
+__device__ __forceinline__ bool w_near(const ComplexDev& c, const Rot& rot, float scan, int gi) {
     const float4 gs = __ldg(c.lgrp + gi);
-    const float R = SCAN_R + gs.w;
+    const float R = scan + gs.w;
     if (!c.rlb || !(R < c.rlb_m)) return true;
     double x, y, z;
     apply(rot, (double)gs.x, (double)gs.y, (double)gs.z, x, y, z);
@@ -1095,7 +1108,7 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(con
         if (lane < 2) W.one[lane] = p.one;
         if (IFACE) W.ibuf[lane] = 0u;   // the slots move with the complex's hash size
         if (lane == 0) {
-            W.rot = pose_matrix(pose_of(p, g));
+            w_pose(W, c, pose_of(p, g));
             if (IFACE) w_iface_begin(W, c, iface_bits(p, c, g));
             else if (c.iface_words) atomicOr(p.status, 2);
         }
@@ -1109,7 +1122,7 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(con
             const int words = min(WD_NEAR, ngrp - g0 + 31) / 32;
             for (int i = wid; i < words; i += NW) {
                 const int gi = g0 + i * 32 + lane;
-                const bool near = gi < ngrp && (((c.flags & F_FAR) && !far_sep) || w_near(c, W.rot, gi));
+                const bool near = gi < ngrp && (((c.flags & F_FAR) && !far_sep) || w_near(c, W.rot, W.scan, gi));
                 const unsigned m = __ballot_sync(0xffffffffu, near);
                 if (lane == 0) s_near[i] = m;
             }
