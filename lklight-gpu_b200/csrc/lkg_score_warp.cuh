@@ -85,7 +85,7 @@ struct __align__(16) WPair {
 template <int G>
 struct WSlots {
     Rot rot;                          // pose of the current work unit
-    float scan;                       // and its search radius around an atom (w_pose)
+    float scan, stretch;              // and its search radius around an atom, its factor on lengths (w_pose)
     WPair pair[G / 2];
     float4 quad[(G + 3) / 4];         // candidate test of each quad's sphere: -2 c', R^2 - |c'|^2 (c' = c - group centre)
     unsigned list[(G + 3) / 4][W_LIST<G> + 16];   // receptor indices of each quad's candidates (and padding)
@@ -275,8 +275,12 @@ __device__ __forceinline__ int w_lane() {
     return (int)l;
 }
 
-// The unit's pose, and the search radius of its atoms: SCAN_R grown by what f32
-// takes from the positions.  The receptor's and the centres' are rounded (2^-24
+// The unit's pose, its factor on lengths, and the search radius of its atoms.
+// A quaternion (w, v) is used as given: the matrix keeps v's axis and turns the
+// plane across it by a matrix of norm sqrt(1 + 4 |v|^2 (|q|^2 - 1)), so the
+// ligand's spheres grow by at most that (1 for unit quaternions to the last place
+// of f32, which the spheres' own margin of 1e-6 holds).  The search radius is
+// SCAN_R grown by what f32 takes from the positions.  The receptor's and the centres' are rounded (2^-24
 // of a coordinate each), as are the distances to the cell rows (under 12
 // roundings of a coordinate; 2^-21 is 8 on the radius, 16 on its square).  1e-4 A
 // at 200 A, and at most 1 A, so that a pose at infinity does not search the whole
@@ -284,7 +288,11 @@ __device__ __forceinline__ int w_lane() {
 template <int G>
 __device__ __forceinline__ void w_pose(WSlots<G>& W, const ComplexDev& c, const double* pq) {
     W.rot = pose_matrix(pq);
-    W.scan = SCAN_R + fminf(0x1p-21f * ((float)(fabs(pq[4]) + fabs(pq[5]) + fabs(pq[6])) + c.lext), 1.f);
+    const double v2 = pq[1] * pq[1] + pq[2] * pq[2] + pq[3] * pq[3];
+    const float e = (float)(4.0 * v2 * (pq[0] * pq[0] + v2 - 1.0));
+    W.stretch = e > 0.f && e < 3e38f ? sqrtf(1.f + e) : 1.f;
+    W.scan = SCAN_R +
+             fminf(0x1p-21f * ((float)(fabs(pq[4]) + fabs(pq[5]) + fabs(pq[6])) + W.stretch * c.lext), 1.f);
 }
 
 // the descriptor of a unit's complex into shared memory by n threads (its
@@ -621,7 +629,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
                 if (lane >= Q0 && lane <= Q0 + NQ) {
                     const float4 s = lane == Q0 + NQ ? __ldg(c.lgrp + grp) : (quad ? __ldg(c.lquad + qi) : make_float4(0.f, 0.f, 0.f, 0.f));
                     b = make_double4((double)s.x, (double)s.y, (double)s.z, 0.0);
-                    rad = W.scan + s.w;
+                    rad = fmaf(W.stretch, s.w, W.scan);
                 }
             };
             if (atom) b = c.lpos64[j];
@@ -1053,11 +1061,12 @@ constexpr int WD_BLOCKS = 3;
 // ligand on a 101,000-atom receptor 84-89 % of the groups of 16)
 constexpr int WD_NEAR = 1024;
 
-// whether a receptor atom can lie within reach of group gi (its sphere grown by
-// `scan`), by the receptor's distance bound at the posed centre
-__device__ __forceinline__ bool w_near(const ComplexDev& c, const Rot& rot, float scan, int gi) {
+// whether a receptor atom can lie within reach of group gi (its sphere, by the
+// pose's factor, grown by `scan`), by the receptor's distance bound at the posed
+// centre
+__device__ __forceinline__ bool w_near(const ComplexDev& c, const Rot& rot, float scan, float stretch, int gi) {
     const float4 gs = __ldg(c.lgrp + gi);
-    const float R = scan + gs.w;
+    const float R = fmaf(stretch, gs.w, scan);
     if (!c.rlb || !(R < c.rlb_m)) return true;
     double x, y, z;
     apply(rot, (double)gs.x, (double)gs.y, (double)gs.z, x, y, z);
@@ -1122,7 +1131,7 @@ __global__ void __launch_bounds__(WD_THREADS, WD_BLOCKS) k_score_warp_desolv(con
             const int words = min(WD_NEAR, ngrp - g0 + 31) / 32;
             for (int i = wid; i < words; i += NW) {
                 const int gi = g0 + i * 32 + lane;
-                const bool near = gi < ngrp && (((c.flags & F_FAR) && !far_sep) || w_near(c, W.rot, W.scan, gi));
+                const bool near = gi < ngrp && (((c.flags & F_FAR) && !far_sep) || w_near(c, W.rot, W.scan, W.stretch, gi));
                 const unsigned m = __ballot_sync(0xffffffffu, near);
                 if (lane == 0) s_near[i] = m;
             }
