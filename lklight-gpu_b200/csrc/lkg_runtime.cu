@@ -354,18 +354,28 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
     }
     // bounding spheres (ligand frame) of every searched group and every
     // quad of 4 consecutive atoms, for the warp kernels' candidate search;
-    // around the f32 centres that the kernels see
+    // around the f32 centres that the kernels see.  An atom without a finite
+    // position is near nothing: the spheres are those of the others
     const int G = ctx->scan();
+    auto placed = [&](int k) {
+        const double* x = &L.c[3 * (size_t)order[k]];
+        return std::isfinite(x[0]) && std::isfinite(x[1]) && std::isfinite(x[2]);
+    };
     auto spheres = [&](int step) {
         std::vector<float4> out(std::max((n + step - 1) / step, 1));
         for (int gi = 0; gi * step < n; ++gi) {
             const int a0 = gi * step, a1 = std::min(n, a0 + step);
             double cen[3] = {0, 0, 0};
-            for (int k = a0; k < a1; ++k)
+            int m = 0;
+            for (int k = a0; k < a1; ++k) {
+                if (!placed(k)) continue;
+                ++m;
                 for (int a = 0; a < 3; ++a) cen[a] += L.c[3 * order[k] + a];
-            for (int a = 0; a < 3; ++a) cen[a] = (float)(cen[a] / (a1 - a0));
+            }
+            for (int a = 0; a < 3; ++a) cen[a] = (float)(cen[a] / std::max(m, 1));
             double r2 = 0;
             for (int k = a0; k < a1; ++k) {
+                if (!placed(k)) continue;
                 double dd = 0;
                 for (int a = 0; a < 3; ++a) dd += (L.c[3 * order[k] + a] - cen[a]) * (L.c[3 * order[k] + a] - cen[a]);
                 r2 = std::max(r2, dd);
