@@ -422,6 +422,9 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
     d.lorig = cr.lorig.as<int>();
     d.lgrp = cr.lgrp.as<float4>();
     d.lquad = cr.lquad.as<float4>();
+    // far groups are skipped by the receptor's distance bound, their share of
+    // the desolvation sum with them: 0 x des, which is 0 only for a finite des
+    d.skip_far = std::all_of(L.des.begin(), L.des.end(), [](double v) { return std::isfinite(v); });
     d.group = G;
     d.ntiles = std::max(1, (n + ctx->tile - 1) / ctx->tile);
     return set_ok();

@@ -1067,7 +1067,7 @@ constexpr int WD_NEAR = 1024;
 __device__ __forceinline__ bool w_near(const ComplexDev& c, const Rot& rot, float scan, float stretch, int gi) {
     const float4 gs = __ldg(c.lgrp + gi);
     const float R = fmaf(stretch, gs.w, scan);
-    if (!c.rlb || !(R < c.rlb_m)) return true;
+    if (!c.rlb || !c.skip_far || !(R < c.rlb_m)) return true;
     double x, y, z;
     apply(rot, (double)gs.x, (double)gs.y, (double)gs.z, x, y, z);
     return !(w_receptor_bound(c, (float)x, (float)y, (float)z) > R);
