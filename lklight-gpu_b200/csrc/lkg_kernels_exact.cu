@@ -27,11 +27,13 @@ static cudaError_t launch_exact_g(const LaunchParams& p, int blocks, cudaStream_
 }
 
 cudaError_t launch_score_exact(const LaunchParams& p, int blocks, cudaStream_t s) {
-    if (p.tile % p.group) return cudaErrorInvalidValue;
+    if (p.atom_elec) return cudaErrorInvalidValue;   // per-atom outputs are k_score_tiles<float>'s
+    if (p.group <= 0 || p.tile % p.group) return cudaErrorInvalidValue;
     switch (p.group) {
         case 4: return launch_exact_g<4>(p, blocks, s);
         case 16: return launch_exact_g<16>(p, blocks, s);
-        default: return launch_exact_g<32>(p, blocks, s);
+        case 32: return launch_exact_g<32>(p, blocks, s);
+        default: return cudaErrorInvalidValue;   // groups of 8 are searched as 16
     }
 }
 
@@ -55,7 +57,8 @@ int max_blocks_score_exact(int group) {
     switch (group) {
         case 4: return occ_exact_g<4>();
         case 16: return occ_exact_g<16>();
-        default: return occ_exact_g<32>();
+        case 32: return occ_exact_g<32>();
+        default: return 0;
     }
 }
 int max_blocks_desolv_exact(int threads, int hcap) {

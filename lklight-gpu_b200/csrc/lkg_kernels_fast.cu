@@ -38,11 +38,12 @@ cudaError_t launch_score_fast(const LaunchParams& p, int threads, int blocks, cu
         k_score_tiles<float><<<blocks, threads, 0, s>>>(p);
         return cudaGetLastError();
     }
-    if (p.tile % p.group) return cudaErrorInvalidValue;
+    if (p.group <= 0 || p.tile % p.group) return cudaErrorInvalidValue;
     switch (p.group) {
         case 4: return launch_warp_g<4>(p, blocks, s);
         case 16: return launch_warp_g<16>(p, blocks, s);
-        default: return launch_warp_g<32>(p, blocks, s);
+        case 32: return launch_warp_g<32>(p, blocks, s);
+        default: return cudaErrorInvalidValue;   // groups of 8 are searched as 16
     }
 }
 
@@ -86,7 +87,8 @@ cudaError_t launch_desolv_fast(const LaunchParams& p, int threads, int blocks, i
     switch (p.group) {
         case 4: return launch_warp_desolv_g<4>(p, blocks, hcap, s);
         case 16: return launch_warp_desolv_g<16>(p, blocks, hcap, s);
-        default: break;
+        case 32: break;
+        default: return cudaErrorInvalidValue;
     }
     size_t sm = desolv_smem_bytes(hcap, false);
     cudaError_t e = cudaFuncSetAttribute(k_score_desolv<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -110,7 +112,8 @@ int max_blocks_score_fast(int /*threads*/, int group) {
     switch (group) {
         case 4: return occ_warp_g<4>();
         case 16: return occ_warp_g<16>();
-        default: return occ_warp_g<32>();
+        case 32: return occ_warp_g<32>();
+        default: return 0;
     }
 }
 int max_blocks_desolv_fast(int threads, int hcap, int group) {

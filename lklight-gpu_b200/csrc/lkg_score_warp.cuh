@@ -918,7 +918,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
 // EXACT: f64 pair math in the reference's operation order
 template <int G, bool IFACE, bool NP, bool STAGE = false, bool EXACT = false>
 __global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCKS) k_score_warp(const __grid_constant__ LaunchParams p) {
-    static_assert(G == 4 || G == 8 || G == 16 || G == 32, "group size");
+    static_assert(G == 4 || G == 16 || G == 32, "group size");
     static_assert(!(STAGE && (IFACE || EXACT)), "the staged variant is the plain kernel's");
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char wk_smem[];
