@@ -1290,19 +1290,39 @@ int lkg_surrogate_create(lkg_ctx* ctx, int complex_id, uint64_t seed, lkg_surrog
     S->cid = complex_id;
     const ComplexRec& cr = *ctx->cx[complex_id];
     // anchors: 16 ligand atoms spread by farthest-point sampling over the
-    // ligand reference coordinates in group order (its first atom is the
-    // first anchor, ties go to the earlier one)
+    // ligand reference coordinates in the order of their bisection into groups
+    // (before the kernels' order inside a group; its first atom is the first
+    // anchor, ties go to the earlier one)
     const int nl = cr.d.nl;
-    std::vector<float4> sorted(nl), lp(nl);
-    cudaMemcpy(sorted.data(), cr.d.lpos, nl * sizeof(float4), cudaMemcpyDeviceToHost);
-    for (int i = 0; i < nl; ++i) lp[i] = sorted[cr.lgroup_order[i]];
+    std::vector<double4> sorted(nl);
+    std::vector<int> orig(nl), order(nl), at(nl);
+    cudaError_t e;
+    if ((e = cudaMemcpy(sorted.data(), cr.d.lpos64, nl * sizeof(double4), cudaMemcpyDeviceToHost)) != cudaSuccess ||
+        (e = cudaMemcpy(orig.data(), cr.d.lorig, nl * sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess) {
+        delete S;
+        return set_error(cuda_to_status(e), "surrogate anchors: %s", cudaGetErrorString(e));
+    }
+    std::vector<double> coord(3 * (size_t)nl);
+    for (int k = 0; k < nl; ++k) {
+        const double4& v = sorted[k];
+        double* x = &coord[3 * (size_t)orig[k]];
+        x[0] = v.x; x[1] = v.y; x[2] = v.z;
+        at[orig[k]] = k;
+        order[k] = k;
+    }
+    bisect_groups(coord.data(), order.data(), nl, ctx->group);
+    std::vector<float4> lp(nl);
+    for (int i = 0; i < nl; ++i) {
+        const double* x = &coord[3 * (size_t)order[i]];
+        lp[i] = make_float4((float)x[0], (float)x[1], (float)x[2], 0.f);
+    }
     std::vector<int> anc;
     std::vector<float> dmin(nl, 1e30f);
     int cur = 0;
     float rmax = 0.f;
     for (int i = 0; i < nl; ++i) rmax = std::max(rmax, std::sqrt(lp[i].x * lp[i].x + lp[i].y * lp[i].y + lp[i].z * lp[i].z));
     for (int a = 0; a < NA; ++a) {
-        anc.push_back(cr.lgroup_order[cur]);
+        anc.push_back(at[order[cur]]);
         int best = 0;
         float bd = -1.f;
         for (int i = 0; i < nl; ++i) {
@@ -1330,7 +1350,6 @@ int lkg_surrogate_create(lkg_ctx* ctx, int complex_id, uint64_t seed, lkg_surrog
         for (size_t i = S->off[2 * L]; i < S->off[2 * L + 1]; ++i) p[i] = (float)((2.0 * u() - 1.0) * lim);
     }
     int rc = 0;
-    cudaError_t e;
     if ((e = S->p.reserve(NPARAM * 4)) != cudaSuccess || (e = S->g.reserve(NPARAM * 4)) != cudaSuccess ||
         (e = S->m1.reserve(NPARAM * 4)) != cudaSuccess || (e = S->m2.reserve(NPARAM * 4)) != cudaSuccess ||
         (e = S->anchors.reserve(NA * sizeof(int))) != cudaSuccess || (e = S->loss.reserve(sizeof(float))) != cudaSuccess ||

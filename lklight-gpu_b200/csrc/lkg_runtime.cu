@@ -180,14 +180,14 @@ std::vector<float> receptor_distance_bound(const double* c, int n, int dims[3], 
 namespace {
 
 // rpk from rpos and rpar (both float4 of an atom side by side), then an atom
-// out of reach of everything that adds nothing (it pads the candidate lists)
+// out of reach of everything that adds nothing (it pads the candidate lists).
+// Queued only: the caller waits for the stream later on
 int interleave_receptor(lkg_ctx* ctx, ComplexRec& cr, int n) {
     LKG_CK(cr.rpk.reserve(((size_t)n + 1) * 2 * sizeof(float4)), "receptor arrays");
     LKG_CK(interleave_atoms(cr.rpos.as<float4>(), cr.rpar.as<float4>(), cr.rsolv64.as<double2>(), n,
                             cr.rpk.as<float4>(), ctx->stream),
            "receptor arrays");
     ctx->launches++;
-    LKG_CK(cudaStreamSynchronize(ctx->stream), "receptor arrays");
     return 0;
 }
 
@@ -300,9 +300,14 @@ int build_receptor(lkg_ctx* ctx, const MolIn& R, ComplexRec& cr) {
     return set_ok();
 }
 
+}  // namespace
+
 // recursive coordinate bisection: order idx[0..n) so that every run of G
 // consecutive atoms (and every run of a power-of-two number of groups) is
-// spatially compact; each split cuts the longest extent at a multiple of G
+// spatially compact; each split cuts the longest extent at a multiple of G.
+// A part that is split again is only partitioned, not sorted (the order inside
+// comes from its own splits; coordinate, then index, is a total order): 5.4 ms
+// for 12,000 atoms in groups of 16 and quads, 9.9 with sorts
 void bisect_groups(const double* c, int* idx, int n, int G) {
     if (n <= G) return;
     double mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -315,14 +320,18 @@ void bisect_groups(const double* c, int* idx, int n, int G) {
     for (int a = 1; a < 3; ++a)
         if (mx[a] - mn[a] > mx[ax] - mn[ax]) ax = a;
     auto key = [&](int u) { const double v = c[3 * u + ax]; return std::isnan(v) ? INFINITY : v; };
-    std::sort(idx, idx + n, [&](int u, int v) {
+    auto before = [&](int u, int v) {
         const double cu = key(u), cv = key(v);
         return cu < cv || (cu == cv && u < v);
-    });
+    };
     const int ng = (n + G - 1) / G, left = (ng / 2) * G;
+    if (left > G && n - left > G) std::nth_element(idx, idx + left, idx + n, before);
+    else std::sort(idx, idx + n, before);   // a group keeps the order it gets here
     bisect_groups(c, idx, left, G);
     bisect_groups(c, idx + left, n - left, G);
 }
+
+namespace {
 
 // ligand: bisection order in the groups that are searched together
 int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
@@ -330,15 +339,9 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
     const int n = L.n;
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
-    std::vector<int> coarse = order;   // in groups of ctx->group (the surrogate's anchors)
-    bisect_groups(L.c.data(), coarse.data(), n, ctx->group);
     bisect_groups(L.c.data(), order.data(), n, ctx->scan());
     for (int k = 0; k < n; k += ctx->scan())   // and quads compact inside each group
         bisect_groups(L.c.data(), order.data() + k, std::min(ctx->scan(), n - k), 4);
-    std::vector<int> at(n);
-    for (int k = 0; k < n; ++k) at[order[k]] = k;
-    cr.lgroup_order.resize(n);
-    for (int k = 0; k < n; ++k) cr.lgroup_order[k] = at[coarse[k]];
     std::vector<float4> pos(n), par(n);
     std::vector<float2> sol(n);
     std::vector<double4> pos64(n), par64(n);
@@ -384,7 +387,7 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
         }
         return out;
     };
-    const std::vector<float4> grp = spheres(G);
+    std::vector<float4> grp = spheres(G);
     std::vector<float4> quad = spheres(4);
     // A quad's test, |a'|^2 - 2 a'.c' <= r^2 - |c'|^2 in f32 relative to the
     // group's centre (r = SCAN_R + radius), is off by at most 18 roundings
@@ -405,9 +408,10 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
         ext2 = std::max(ext2, dd);
     }
     d.lext = (float)(std::sqrt(3.0 * ext2) * (1.0 + 1e-6));
+    const size_t ngrp = grp.size();
+    grp.insert(grp.end(), quad.begin(), quad.end());
     cudaStream_t s = ctx->stream;
     LKG_CK(upload(cr.lgrp, grp, s), "upload ligand");
-    LKG_CK(upload(cr.lquad, quad, s), "upload ligand");
     LKG_CK(upload(cr.lpos, pos, s), "upload ligand");
     LKG_CK(upload(cr.lpar, par, s), "upload ligand");
     LKG_CK(upload(cr.lsolv, sol, s), "upload ligand");
@@ -421,7 +425,7 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
     d.lpos64 = cr.lpos64.as<double4>(); d.lpar64 = cr.lpar64.as<double4>(); d.lsolv64 = cr.lsolv64.as<double2>();
     d.lorig = cr.lorig.as<int>();
     d.lgrp = cr.lgrp.as<float4>();
-    d.lquad = cr.lquad.as<float4>();
+    d.lquad = d.lgrp + ngrp;
     // far groups are skipped by the receptor's distance bound, their share of
     // the desolvation sum with them: 0 x des, which is 0 only for a finite des
     d.skip_far = std::all_of(L.des.begin(), L.des.end(), [](double v) { return std::isfinite(v); });
@@ -527,7 +531,9 @@ static int set_rpar_tag_signs(lkg_ctx* ctx, ComplexRec& cr, const std::vector<in
         par[k].z = tagged ? -std::fabs(par[k].z) : std::fabs(par[k].z);
     }
     LKG_CK(to_device(cr.rpar.p, par.data(), nr * sizeof(float4), ctx->stream), "receptor tags");
-    return interleave_receptor(ctx, cr, nr);
+    if (const int st = interleave_receptor(ctx, cr, nr)) return st;
+    LKG_CK(cudaStreamSynchronize(ctx->stream), "receptor tags");
+    return 0;
 }
 
 int complex_set_ligand(lkg_ctx* ctx, int id, const MolIn& lig) {

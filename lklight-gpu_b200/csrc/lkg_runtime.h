@@ -81,11 +81,7 @@ struct ComplexRec {
     int family = -1;
     DBuf rpos, rpar, rpk, rsolv, rpos64, rpar64, rsolv64, rorig, cell_start;
     DBuf rlb;   // distance lower bound of the receptor (ComplexDev::rlb)
-    DBuf lpos, lpar, lsolv, lpos64, lpar64, lsolv64, lorig, lgrp, lquad;
-    // the ligand's atoms (kernel indices) in the order of the bisection into
-    // groups, before each group was bisected into quads: the surrogate's
-    // anchors are sampled in this order
-    std::vector<int> lgroup_order;
+    DBuf lpos, lpar, lsolv, lpos64, lpar64, lsolv64, lorig, lgrp;   // (lgrp: the groups' spheres, then the quads')
     DBuf phi;
     DBuf rtag, ltag;   // interface tags (restraints / membrane), when set
     ComplexDev d{};
@@ -190,6 +186,9 @@ int build_receptor_device(lkg_ctx* ctx, const MolIn& R, ComplexRec& cr, const fl
 // that adds nothing (ComplexDev::rpk; out: 2 (n + 1) float4)
 cudaError_t interleave_atoms(const float4* pos, const float4* par, const double2* solv, int n, float4* out,
                              cudaStream_t s);
+// recursive coordinate bisection of idx[0..n) into groups of G atoms (c: x, y, z
+// by atom)
+void bisect_groups(const double* c, int* idx, int n, int G);
 // replace the ligand of an existing complex (cuda_full_score)
 int complex_set_ligand(lkg_ctx* ctx, int id, const MolIn& lig);
 // a complex changed: descriptors to upload, captured graphs out of date
