@@ -1174,7 +1174,8 @@ static int score_host(lkg_ctx* ctx, int id, int n, const double* poses, double* 
     double* d_iface = iface ? (double*)(ctx->d_parts.as<char>() + qb) : nullptr;
     if (iface) LKG_CK(cudaMemsetAsync(d_iface, 0, ib, ctx->stream), "interface output");
     st = launch_items(ctx, 1, &id, &n, ctx->d_poses.as<double>(), ctx->d_scores.as<double>(),
-                      parts ? ctx->d_parts.as<double>() : nullptr, 0, 0, nullptr, nullptr, d_iface, status);
+                      parts ? ctx->d_parts.as<double>() : nullptr, 0, 0, nullptr, nullptr, d_iface, status,
+                      in_launch ? poses : nullptr);
     if (st) return st;
     LKG_CK(cudaMemcpyAsync(ctx->h_out.p, ctx->d_scores.p, ob, cudaMemcpyDeviceToHost, ctx->stream), "score readback");
     if (parts)
