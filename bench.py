@@ -41,9 +41,9 @@ REPO = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, REPO)
 
 FLOPS_PER_PAIR = {"dna": 24, "pydock": 23, "vdw": 19, "cpydock": 25}
-# DRAM bytes per pose of the fast kernel (56.8 MB per 24,000-pose launch of
+# DRAM bytes per pose of the fast kernel (62.6 MB per 24,000-pose launch of
 # the 4-complex profiling case under ncu, at tile 256, groups of 16, cell 7 A)
-TRAFFIC_PER_POSE = 56.8e6 / 24000
+TRAFFIC_PER_POSE = 62.6e6 / 24000
 FAR_FLOPS = 30
 
 

@@ -318,7 +318,7 @@ int lkg_surrogate_status(lkg_surrogate* s, int* bits);
 int lkg_field_build(const double* coords, const double* charges, int32_t n,
                     double origin[3], int32_t dims[3], double* spacing, float* phi);
 /* Lower bound of the distance from each of m points (x, y, z) to the
- * nearest of n receptor atoms, as the warp kernels use it to skip ligand
+ * nearest of n receptor atoms, as the cpydock kernel uses it to skip ligand
  * groups that no receptor atom can reach (a 2 A grid over the receptor's
  * box grown by 24 A; 24 outside it).  No counterpart in the reference. */
 int lkg_receptor_distance_bound(const double* coords, int32_t n, const double* points, int32_t m, float* out);

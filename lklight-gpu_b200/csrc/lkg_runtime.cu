@@ -89,8 +89,8 @@ cudaError_t upload(DBuf& b, const std::vector<T>& v, cudaStream_t s) {
 // exact squared Euclidean distance transform over the cell centres (three
 // separable passes of the lower envelope of parabolas, Felzenszwalb and
 // Huttenlocher, "Distance transforms of sampled functions", 2012).  A point
-// outside the grid is farther than RLB_M from every atom.  The warp kernels
-// skip a ligand group whose centre's bound exceeds its candidate radius.
+// outside the grid is farther than RLB_M from every atom.  The cpydock
+// kernel skips a ligand group whose centre's bound exceeds its candidate radius.
 constexpr float RLB_S = 2.0f, RLB_M = 24.0f;
 constexpr size_t RLB_MAX_CELLS = (size_t)1 << 26;   // 256 MB of bound at most
 
@@ -197,7 +197,7 @@ int interleave_receptor(lkg_ctx* ctx, ComplexRec& cr, int n) {
 int build_receptor(lkg_ctx* ctx, const MolIn& R, ComplexRec& cr) {
     ComplexDev& d = cr.d;
     const int n = R.n;
-    // the warp kernel's hit queue packs a receptor index into 26 bits
+    // the warp kernels pack a receptor index into 26 bits beside a slot
     if (n >= (1 << 26)) return set_error(LKG_ERR_ARG, "receptor has %d atoms (limit %d)", n, (1 << 26) - 1);
     // grid shape: the caller's, else per kernel: the warp kernels enumerate
     // rows per ligand group (coarser rows, finer x trim pay off); cpydock
@@ -271,7 +271,7 @@ int build_receptor(lkg_ctx* ctx, const MolIn& R, ComplexRec& cr) {
     d.rorig = cr.rorig.as<int>(); d.cell_start = cr.cell_start.as<int>();
     d.ncx = nc[0]; d.ncy = nc[1]; d.ncz = nc[2];
     d.ox = o[0]; d.oy = o[1]; d.oz = o[2]; d.h = h; d.inv_h = inv_h; d.hx = hx; d.inv_hx = inv_hx;
-    {   // the distance bound the warp kernels skip far ligand groups with
+    {   // the distance bound the cpydock kernel skips far ligand groups with
         int ld[3];
         float lo[3];
         const std::vector<float> lb = receptor_distance_bound(R.c.data(), n, ld, lo);
@@ -1434,7 +1434,7 @@ int lkg_plan_sync(lkg_plan* P) {
 extern "C" {
 
 // The lower bound of the distance to the nearest of n receptor atoms that
-// the warp kernels skip far ligand groups with, at m points (host; for
+// the cpydock kernel skips far ligand groups with, at m points (host; for
 // checks of the bound).
 int lkg_receptor_distance_bound(const double* coords, int32_t n, const double* points, int32_t m, float* out) {
     if (n < 0 || m < 0 || (n > 0 && !coords) || (m > 0 && (!points || !out)))

@@ -1,14 +1,15 @@
-// Warp-independent fused scorer (f32 fast path, dna / pydock / vdw and the
-// reference-compatible flag combinations).
+// Warp-independent fused scorer: dna / pydock / vdw and the
+// reference-compatible flag combinations in both precisions (f32 pair math, or
+// EXACT: f64 in the reference's operation order), and the fast cpydock kernel.
 //
 // Every warp fetches its own work units from the global counter; there is
 // no block-level barrier inside the loop, so a warp that meets a crowded
 // interface never holds up the warps beside it.  A work unit is a tile of
-// `p.tile` ligand atoms of one pose, split into groups of G consecutive
-// atoms (spatially compact: the ligand is ordered by recursive coordinate
-// bisection in groups of G) whose bounding sphere (centre, radius rho, in the
-// ligand frame) is computed on the host, as is the sphere of every quad of 4
-// consecutive atoms.  Per group:
+// `p.tile` ligand atoms of one pose, in small launches a part of one (`p.sub`
+// groups), in groups of G consecutive atoms (spatially compact: the ligand is
+// ordered by recursive coordinate bisection in groups of G) whose bounding
+// sphere (centre, radius rho, in the ligand frame) is computed on the host, as
+// is the sphere of every quad of 4 consecutive atoms.  Per group:
 //   1. lanes 0..G-1 transform their atom in f64 (kept as an f32 value plus
 //      the rounding residual), add the far-field term q * phi(x'), and park
 //      position and parameters in shared memory, two neighbouring atoms
@@ -41,11 +42,12 @@ constexpr int WK_THREADS = 128;   // 4 independent warps per block
 
 // candidates a quad's list holds: lists are scored when one holds more than
 // W_LIST - 64 (two chunks add at most 64).  Long enough that most groups are
-// scored once, at their end, short enough to leave L1 its room.  ms at 96 / 128
-// / 192 / 256 / 384 / 512: 1800 vdw poses with groups of 8: 0.89 / 0.85 / 0.83
-// / 0.80 / 0.81 / 0.84; sixteen complexes with groups of 16: 13.0 / 12.1 / 11.9
-// / 12.0 / 12.5 / 15.6.
-template <int G> constexpr int W_LIST = G <= 8 ? 256 : 192;
+// scored once, at their end, short enough to leave L1 its room.  3000 vdw poses
+// of a 1300-atom ligand on 12,600 atoms at protein density, ms at 128 / 160 /
+// 192 / 256 / 384: groups of 4 (one list): 2.94 / 2.89 / 2.84 / 2.80 / 2.76;
+// groups of 16 (four): 2.04 / 1.99 / 2.00 / 2.02 / 2.18; groups of 32 (eight):
+// 2.35 / 2.45 / 2.41 / 2.65 / 3.59.
+template <int G> constexpr int W_LIST = G == 4 ? 256 : 192;
 
 // resident blocks per SM the register budget is sized for: 72 registers (a
 // few spills in the cold parts).  Sixteen complexes of 2,000 poses: 12.5 ms at
