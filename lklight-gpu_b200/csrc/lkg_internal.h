@@ -58,10 +58,10 @@ struct ComplexDev {
     const float* rlb;
     int rlbx, rlby, rlbz;
     float rlbox, rlboy, rlboz, rlb_inv, rlb_m;
-    int skip_far;            // ligand groups out of the receptor's reach add nothing (cpydock kernel)
     const float4* lgrp;      // per group of `group` atoms: ligand-frame centre, radius
     const float4* lquad;     // per 4 consecutive atoms: ligand-frame centre, radius (with what its test needs, build_ligand)
     float lext;              // |x| + |y| + |z| of a ligand atom in any rotation is at most this (before any stretch)
+    int skip_far;            // groups out of the receptor's reach add nothing (cpydock kernel)
     int group;               // ligand atoms per candidate-search group
     int ntiles;              // ceil(nl / tile)
     // far field: fnx x fny x fnz points in bricks of 4 x 4 x 4 (fbx x fby x

@@ -10,6 +10,13 @@ static size_t exact_smem() {
     return (size_t)(WK_THREADS / 32) * (sizeof(WSlots<G>) + sizeof(ComplexDev) + sizeof(WExact<G>));
 }
 
+// WK_BLOCKS_EXACT blocks (1 KB more each, in units of 128 bytes) within the
+// largest shared-memory share but one: beyond it the SM's L1 halves, and 200
+// dna poses take 356 us instead of 335
+static_assert(((((WK_THREADS / 32) * (sizeof(WSlots<16>) + sizeof(ComplexDev) + sizeof(WExact<16>)) + 1024) + 127) / 128) *
+                      128 * WK_BLOCKS_EXACT <= 196 * 1024,
+              "the f64 kernel's shared memory leaves L1 its room");
+
 template <int G, bool IFACE, bool NP>
 static cudaError_t launch_exact_gi(const LaunchParams& p, int blocks, cudaStream_t s) {
     const size_t sm = exact_smem<G>();
