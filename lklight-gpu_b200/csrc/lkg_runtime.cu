@@ -383,7 +383,7 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
                 for (int a = 0; a < 3; ++a) dd += (L.c[3 * order[k] + a] - cen[a]) * (L.c[3 * order[k] + a] - cen[a]);
                 r2 = std::max(r2, dd);
             }
-            out[gi] = make_float4((float)cen[0], (float)cen[1], (float)cen[2], (float)(std::sqrt(r2) * (1.0 + 1e-6) + 1e-3));
+            out[gi] = make_float4((float)cen[0], (float)cen[1], (float)cen[2], (float)(std::sqrt(r2) * (1.0 + 4e-6) + 1e-3));
         }
         return out;
     };

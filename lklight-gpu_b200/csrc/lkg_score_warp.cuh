@@ -280,9 +280,9 @@ __device__ __forceinline__ int w_lane() {
 // The unit's pose, its factor on lengths, and the search radius of its atoms.
 // A quaternion (w, v) is used as given: the matrix keeps v's axis and turns the
 // plane across it by a matrix of norm sqrt(1 + 4 |v|^2 (|q|^2 - 1)), so the
-// ligand's spheres grow by at most that (1 for unit quaternions to the last place
-// of f32, which the spheres' own margin of 1e-6 holds).  The search radius is
-// SCAN_R grown by what f32 takes from the positions.  The receptor's and the centres' are rounded (2^-24
+// ligand's spheres grow by at most that: up to 2e-6 (the f32 arithmetic here is
+// off by 1e-6 at most near unit quaternions) by the spheres' own margin of 4e-6.
+// The search radius is SCAN_R grown by what f32 takes from the positions.  The receptor's and the centres' are rounded (2^-24
 // of a coordinate each), as are the distances to the cell rows (under 12
 // roundings of a coordinate; 2^-21 is 8 on the radius, 16 on its square).  1e-4 A
 // at 200 A, and at most 1 A, so that a pose at infinity does not search the whole
@@ -290,11 +290,13 @@ __device__ __forceinline__ int w_lane() {
 template <int G>
 __device__ __forceinline__ void w_pose(WSlots<G>& W, const ComplexDev& c, const double* pq) {
     W.rot = pose_matrix(pq);
-    const double v2 = pq[1] * pq[1] + pq[2] * pq[2] + pq[3] * pq[3];
-    const float e = (float)(4.0 * v2 * (pq[0] * pq[0] + v2 - 1.0));
-    W.stretch = e > 0.f && e < 3e38f ? sqrtf(1.f + e) : 1.f;
-    W.scan = SCAN_R +
-             fminf(0x1p-21f * ((float)(fabs(pq[4]) + fabs(pq[5]) + fabs(pq[6])) + W.stretch * c.lext), 1.f);
+    const float qw = (float)pq[0], qx = (float)pq[1], qy = (float)pq[2], qz = (float)pq[3];
+    const float v2 = qx * qx + qy * qy + qz * qz, e = 4.f * v2 * (qw * qw + v2 - 1.f);
+    float s = 1.f;
+    if (e > 4e-6f && e < 3e38f) s = sqrtf(1.f + e);
+    W.stretch = s;
+    const float t = fabsf((float)pq[4]) + fabsf((float)pq[5]) + fabsf((float)pq[6]);
+    W.scan = SCAN_R + fminf(0x1p-21f * (t + s * c.lext), 1.f);
 }
 
 // the descriptor of a unit's complex into shared memory by n threads (its
