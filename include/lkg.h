@@ -151,8 +151,8 @@ int lkg_ctx_set_precision(lkg_ctx* ctx, int precision);
  * complexes with groups of 32); 0 keeps the current value. */
 int lkg_ctx_set_tiles(lkg_ctx* ctx, int threads_per_block, int cell_size_milli_angstrom);
 /* Ligand atoms per candidate-search group of the warp kernel (4, 8, 16 or
- * 32; default 8, two of which are searched together); fixed once complexes
- * exist. */
+ * 32; default 8, two of which are searched together but for cpydock ligands
+ * of up to 700 atoms); fixed once complexes exist. */
 int lkg_ctx_set_group(lkg_ctx* ctx, int group);
 /* x sub-cells per receptor cell edge (1..8; default 8, 4 for cpydock
  * complexes with groups of 32): the near scan trims each (z, y) cell row to

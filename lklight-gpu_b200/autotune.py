@@ -17,12 +17,15 @@ import os
 
 import numpy as np
 
-# (groups of 8 are searched two at a time, as groups of 16: the same kernel shape)
 CANDIDATES = [
     (128, 16, 4.0, 8), (128, 16, 5.0, 8), (128, 16, 6.0, 8), (128, 16, 7.0, 8),
     (128, 16, 8.0, 8), (256, 16, 6.0, 8), (256, 16, 7.0, 8), (256, 16, 8.0, 8), (128, 32, 6.0, 8), (256, 32, 7.0, 8),
     (128, 4, 4.0, 8), (64, 16, 4.0, 8),
 ]
+# groups of 8 are searched two at a time, as groups of 16 (the same kernel
+# shape), but for cpydock ligands of up to 700 atoms: batches with one also try
+SMALL_CPYDOCK = 700
+CANDIDATES_SMALL_CPYDOCK = [(128, 8, 4.0, 8), (128, 8, 5.0, 8), (128, 8, 6.0, 8), (128, 8, 7.0, 8)]
 DEFAULT_CACHE = os.path.join(os.path.expanduser("~"), ".cache", "lkg", "tuning.json")
 
 
@@ -56,7 +59,12 @@ def _sample(items, k):
     return picks
 
 
-def autotune(items, device=0, candidates=CANDIDATES, sample=12, poses_per_complex=3000, reps=3,
+def candidates_for(items):
+    small = any(it["family"] == "cpydock" and len(it["lig"]["coords"]) <= SMALL_CPYDOCK for it in items)
+    return CANDIDATES + (CANDIDATES_SMALL_CPYDOCK if small else [])
+
+
+def autotune(items, device=0, candidates=None, sample=12, poses_per_complex=3000, reps=3,
              cache_path=DEFAULT_CACHE, verbose=False):
     """Returns dict(tile, group, cell, xsub, ms, source) for a batch given as
     a list of dicts with ``family``, ``rec``, ``lig`` and ``poses`` (N x 7,
@@ -84,7 +92,7 @@ def autotune(items, device=0, candidates=CANDIDATES, sample=12, poses_per_comple
         d_poses = torch.tensor(poses, dtype=torch.float64, device="cuda")
         d_scores = torch.zeros(len(poses), dtype=torch.float64, device="cuda")
         results = []
-        for tile, group, cell, xsub in candidates:
+        for tile, group, cell, xsub in candidates or candidates_for(items):
             ctx = lkg.Context(device=device, tile=tile, group=group, cell=cell, xsub=xsub)
             try:
                 ids = [ctx.add_complex(it["family"], it["rec"], it["lig"]) for it in sub]

@@ -86,6 +86,7 @@ cudaError_t launch_far_poses(const LaunchParams& p, int blocks, cudaStream_t s) 
 cudaError_t launch_desolv_fast(const LaunchParams& p, int threads, int blocks, int hcap, cudaStream_t s) {
     switch (p.group) {
         case 4: return launch_warp_desolv_g<4>(p, blocks, hcap, s);
+        case 8: return launch_warp_desolv_g<8>(p, blocks, hcap, s);
         case 16: return launch_warp_desolv_g<16>(p, blocks, hcap, s);
         case 32: break;
         default: return cudaErrorInvalidValue;
@@ -119,6 +120,7 @@ int max_blocks_score_fast(int /*threads*/, int group) {
 int max_blocks_desolv_fast(int threads, int hcap, int group) {
     switch (group) {
         case 4: return occ_warp_desolv_g<4>(hcap);
+        case 8: return occ_warp_desolv_g<8>(hcap);
         case 16: return occ_warp_desolv_g<16>(hcap);
         default: break;
     }

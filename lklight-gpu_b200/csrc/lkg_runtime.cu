@@ -334,14 +334,14 @@ void bisect_groups(const double* c, int* idx, int n, int G) {
 namespace {
 
 // ligand: bisection order in the groups that are searched together
-int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
+int build_ligand(lkg_ctx* ctx, const MolIn& L, unsigned flags, ComplexRec& cr) {
     ComplexDev& d = cr.d;
-    const int n = L.n;
+    const int n = L.n, G = ctx->scan(flags & F_DESOLV, L.n);
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
-    bisect_groups(L.c.data(), order.data(), n, ctx->scan());
-    for (int k = 0; k < n; k += ctx->scan())   // and quads compact inside each group
-        bisect_groups(L.c.data(), order.data() + k, std::min(ctx->scan(), n - k), 4);
+    bisect_groups(L.c.data(), order.data(), n, G);
+    for (int k = 0; k < n; k += G)   // and quads compact inside each group
+        bisect_groups(L.c.data(), order.data() + k, std::min(G, n - k), 4);
     std::vector<float4> pos(n), par(n);
     std::vector<float2> sol(n);
     std::vector<double4> pos64(n), par64(n);
@@ -359,7 +359,6 @@ int build_ligand(lkg_ctx* ctx, const MolIn& L, ComplexRec& cr) {
     // quad of 4 consecutive atoms, for the warp kernels' candidate search;
     // around the f32 centres that the kernels see.  An atom without a finite
     // position is near nothing: the spheres are those of the others
-    const int G = ctx->scan();
     auto placed = [&](int k) {
         const double* x = &L.c[3 * (size_t)order[k]];
         return std::isfinite(x[0]) && std::isfinite(x[1]) && std::isfinite(x[2]);
@@ -486,13 +485,13 @@ int build_field(lkg_ctx* ctx, const MolIn& R, const lkg_field* f, bool build, Co
     return set_ok();
 }
 
-int occupancy(lkg_ctx* ctx, bool desolv, bool exact, int threads, int hcap) {
-    Occupancy& o = desolv ? ctx->occ_desolv[exact] : ctx->occ_tiles[exact];
-    if (o.threads == threads && o.hcap == hcap && o.blocks > 0) return o.blocks;
+int occupancy(lkg_ctx* ctx, bool desolv, bool exact, int threads, int hcap, int group) {
+    Occupancy& o = desolv ? ctx->occ_desolv[exact][group == 8] : ctx->occ_tiles[exact];
+    if (o.threads == threads && o.hcap == hcap && o.group == group && o.blocks > 0) return o.blocks;
     int b;
-    if (desolv) b = exact ? max_blocks_desolv_exact(threads, hcap) : max_blocks_desolv_fast(threads, hcap, ctx->scan());
-    else b = exact ? max_blocks_score_exact(ctx->scan()) : max_blocks_score_fast(threads, ctx->scan());
-    o.threads = threads; o.hcap = hcap; o.blocks = std::max(1, b);
+    if (desolv) b = exact ? max_blocks_desolv_exact(threads, hcap) : max_blocks_desolv_fast(threads, hcap, group);
+    else b = exact ? max_blocks_score_exact(group) : max_blocks_score_fast(threads, group);
+    o.threads = threads; o.hcap = hcap; o.group = group; o.blocks = std::max(1, b);
     return o.blocks;
 }
 
@@ -506,7 +505,7 @@ int complex_create(lkg_ctx* ctx, int family, unsigned flags, int lj_form, const 
     cr->family = family;
     int st;
     if ((st = build_receptor(ctx, rec, *cr))) return st;
-    if ((st = build_ligand(ctx, lig, *cr))) return st;
+    if ((st = build_ligand(ctx, lig, flags, *cr))) return st;
     if ((st = build_field(ctx, rec, field, build_field_flag && (flags & F_FAR), *cr))) return st;
     cr->d.flags = flags;
     cr->d.lj_form = lj_form;
@@ -539,7 +538,7 @@ static int set_rpar_tag_signs(lkg_ctx* ctx, ComplexRec& cr, const std::vector<in
 int complex_set_ligand(lkg_ctx* ctx, int id, const MolIn& lig) {
     if (id < 0 || id >= (int)ctx->cx.size()) return set_error(LKG_ERR_ARG, "bad complex id %d", id);
     ComplexRec& cr = *ctx->cx[id];
-    int st = build_ligand(ctx, lig, cr);
+    int st = build_ligand(ctx, lig, cr.d.flags, cr);
     // interface tags refer to the old ligand's atoms
     if (!st && cr.d.iface_words && (st = set_rpar_tag_signs(ctx, cr, nullptr))) return st;
     cr.d.rtag = nullptr; cr.d.ltag = nullptr;
@@ -689,41 +688,54 @@ void Group::pack(char* dst) const {
 constexpr int SPLIT_UNITS = 2;
 static void split_tiles(lkg_ctx* ctx, Group& G) {
     if (G.ic.empty()) return;
-    const long long want = SPLIT_UNITS * (long long)ctx->sm_count * occupancy(ctx, false, false, ctx->tile, 0) *
+    const long long want = SPLIT_UNITS * (long long)ctx->sm_count * occupancy(ctx, false, false, ctx->tile, 0, G.group) *
                            (128 / 32);
-    int sub = ctx->tile / ctx->scan();
+    const int scan = G.group;
+    int sub = ctx->tile / scan;
     auto units = [&](int s) {
         long long n = 0;
         for (size_t i = 0; i < G.ic.size(); ++i) {
-            const long long ng = (ctx->cx[G.ic[i]]->d.nl + ctx->scan() - 1) / ctx->scan();
+            const long long ng = (ctx->cx[G.ic[i]]->d.nl + scan - 1) / scan;
             n += G.inp[i] * ((ng + s - 1) / s);
         }
         return n;
     };
     while (sub > 1 && units(sub) < want) sub >>= 1;
-    if (sub == ctx->tile / ctx->scan()) return;
+    if (sub == ctx->tile / scan) return;
     G.sub = sub;
     for (size_t i = 0; i < G.ic.size(); ++i) {
-        const long long ng = (ctx->cx[G.ic[i]]->d.nl + ctx->scan() - 1) / ctx->scan();
+        const long long ng = (ctx->cx[G.ic[i]]->d.nl + scan - 1) / scan;
         G.ws.push_back(G.ws.back() + G.inp[i] * ((ng + sub - 1) / sub));
         G.g0.push_back(G.g0.back() + G.inp[i] * ng);
     }
 }
 
-int build_groups(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, Group g[2], size_t* n_poses) {
+// the tables of all launch groups, each from a 256-byte boundary (off)
+static std::vector<char> pack_groups(const Group g[N_GROUPS], size_t off[N_GROUPS]) {
+    size_t n = 0;
+    for (int k = 0; k < N_GROUPS; ++k) {
+        off[k] = n;
+        n += (g[k].bytes() + 255) & ~(size_t)255;
+    }
+    std::vector<char> packed(n, 0);
+    for (int k = 0; k < N_GROUPS; ++k) g[k].pack(packed.data() + off[k]);
+    return packed;
+}
+
+int build_groups(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, Group g[N_GROUPS], size_t* n_poses) {
     for (int i = 0; i < n_items; ++i) {
         if (ids[i] < 0 || ids[i] >= (int)ctx->cx.size()) return set_error(LKG_ERR_ARG, "bad complex id %d", ids[i]);
         if (counts[i] < 0) return set_error(LKG_ERR_ARG, "negative pose count");
     }
-    g[0] = Group();
-    g[1] = Group();
-    g[1].kind = 1;
+    for (int k = 0; k < N_GROUPS; ++k) g[k] = Group();
+    g[1].kind = g[2].kind = 1;
     long long pose0 = 0;
     for (int i = 0; i < n_items; ++i) {
         const ComplexDev& d = ctx->cx[ids[i]]->d;
-        const int k = (d.flags & F_DESOLV) ? 1 : 0;
+        const int k = !(d.flags & F_DESOLV) ? 0 : (d.group == 8 ? 2 : 1);
         if (counts[i] > 0) {
             Group& G = g[k];
+            G.group = d.group;
             G.ic.push_back(ids[i]);
             G.ip0.push_back((int)pose0);
             G.inp.push_back(counts[i]);
@@ -734,11 +746,12 @@ int build_groups(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, G
                 while (sc <= d.nr) sc <<= 1;
                 G.spill_cap = std::max(G.spill_cap, sc);
             }
-            // one stride for both groups: a pose's bits sit at pose * stride
-            g[0].iface_words = g[1].iface_words = std::max(g[0].iface_words, d.iface_words);
+            // one stride for all groups: a pose's bits sit at pose * stride
+            g[0].iface_words = std::max(g[0].iface_words, d.iface_words);
         }
         pose0 += counts[i];
     }
+    g[1].iface_words = g[2].iface_words = g[0].iface_words;
     *n_poses = (size_t)pose0;
     split_tiles(ctx, g[0]);
     return set_ok();
@@ -748,8 +761,8 @@ long long group_blocks(lkg_ctx* ctx, const Group& G, bool exact) {
     const bool split = G.sub > 0;
     const long long work = std::max(1LL, split ? G.ws.back() : G.w0.back());
     long long blocks;
-    if (G.kind == 0) blocks = (long long)ctx->sm_count * occupancy(ctx, false, exact, ctx->tile, 0);
-    else blocks = (long long)ctx->sm_count * occupancy(ctx, true, exact, ctx->desolv_threads, G.hcap);
+    if (G.kind == 0) blocks = (long long)ctx->sm_count * occupancy(ctx, false, exact, ctx->tile, 0, G.group);
+    else blocks = (long long)ctx->sm_count * occupancy(ctx, true, exact, ctx->desolv_threads, G.hcap, G.group);
     return std::max(1LL, std::min(blocks, work));
 }
 
@@ -775,7 +788,7 @@ int launch_group(lkg_ctx* ctx, const Group& G, const char* db, Scratch& sc, cons
     p.n_items = ni;
     p.total_work = split ? G.ws.back() : G.w0.back();
     p.tile = ctx->tile;
-    p.group = ctx->scan();
+    p.group = G.group;
     p.poses = d_poses;
     if (h_poses) {
         p.n_param = n_host;
@@ -846,7 +859,7 @@ int launch_items(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, c
                  double* d_scores, double* d_parts, int raw_pairs, int solv_only, float* atom_e,
                  float* atom_v, double* d_iface, int* host_status, const double* h_poses) {
     if (n_items <= 0) return set_ok();
-    Group g[2];
+    Group g[N_GROUPS];
     size_t n_poses = 0;
     int st;
     if ((st = build_groups(ctx, n_items, ids, counts, g, &n_poses))) return st;
@@ -854,23 +867,21 @@ int launch_items(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, c
     if ((st = sync_descriptors(ctx))) return st;
     const size_t units = std::max<size_t>(g[0].partials(), 1);
     LKG_CK(ctx->scratch.ensure(units, n_poses, ctx->stream, n_poses * (size_t)g[0].iface_words), "scratch");
-    const size_t b0 = (g[0].bytes() + 255) & ~(size_t)255, b1 = (g[1].bytes() + 255) & ~(size_t)255;
-    std::vector<char> packed(b0 + b1, 0);
-    g[0].pack(packed.data());
-    g[1].pack(packed.data() + b0);
+    size_t off[N_GROUPS];
+    std::vector<char> packed = pack_groups(g, off);
     if (packed != ctx->last_items || !ctx->d_items.p) {
         // new tables: the previous upload may still be reading the staging buffer
         LKG_CK(cudaStreamSynchronize(ctx->stream), "item staging");
-        LKG_CK(ctx->h_items.reserve(b0 + b1), "item staging");
-        LKG_CK(ctx->d_items.reserve(b0 + b1), "item staging");
-        memcpy(ctx->h_items.p, packed.data(), b0 + b1);
-        LKG_CK(cudaMemcpyAsync(ctx->d_items.p, ctx->h_items.p, b0 + b1, cudaMemcpyHostToDevice, ctx->stream),
+        LKG_CK(ctx->h_items.reserve(packed.size()), "item staging");
+        LKG_CK(ctx->d_items.reserve(packed.size()), "item staging");
+        memcpy(ctx->h_items.p, packed.data(), packed.size());
+        LKG_CK(cudaMemcpyAsync(ctx->d_items.p, ctx->h_items.p, packed.size(), cudaMemcpyHostToDevice, ctx->stream),
                "item upload");
         ctx->last_items.swap(packed);
     }
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < N_GROUPS; ++k) {
         if (g[k].ic.empty()) continue;
-        st = launch_group(ctx, g[k], ctx->d_items.as<char>() + (k ? b0 : 0), ctx->scratch, d_poses, d_scores, d_parts,
+        st = launch_group(ctx, g[k], ctx->d_items.as<char>() + off[k], ctx->scratch, d_poses, d_scores, d_parts,
                           raw_pairs, solv_only, atom_e, atom_v, nullptr, d_iface, host_status, h_poses, (int)n_poses);
         if (st) return st;
     }
@@ -1291,8 +1302,8 @@ int lkg_field_build(const double* coords, const double* charges, int32_t n, doub
 // ---------------------------------------------------------------------------
 struct lkg_plan {
     lkg_ctx* ctx = nullptr;
-    lkg::Group g[2];
-    size_t b0 = 0, n_poses = 0;
+    lkg::Group g[lkg::N_GROUPS];
+    size_t off[lkg::N_GROUPS] = {}, n_poses = 0;
     lkg::DBuf d_tables;
     lkg::Scratch scratch;
     cudaGraph_t graph = nullptr;
@@ -1312,18 +1323,16 @@ int lkg_plan_create(lkg_ctx* ctx, int n_items, const int* ids, const int* counts
     int st = build_groups(ctx, n_items, ids, counts, P->g, &P->n_poses);
     if (!st) st = sync_descriptors(ctx);
     if (st) { delete P; return st; }
-    const size_t b0 = (P->g[0].bytes() + 255) & ~(size_t)255, b1 = (P->g[1].bytes() + 255) & ~(size_t)255;
-    std::vector<char> packed(b0 + b1, 0);
-    P->g[0].pack(packed.data());
-    P->g[1].pack(packed.data() + b0);
-    P->b0 = b0;
+    const std::vector<char> packed = pack_groups(P->g, P->off);
+    size_t spill = 0;
+    for (const Group& G : P->g)
+        spill = std::max({spill, group_spill_bytes(ctx, G, false), group_spill_bytes(ctx, G, true)});
     cudaError_t e;
-    if ((e = P->d_tables.reserve(b0 + b1)) != cudaSuccess ||
-        (e = to_device(P->d_tables.p, packed.data(), b0 + b1, ctx->stream)) != cudaSuccess ||
+    if ((e = P->d_tables.reserve(packed.size())) != cudaSuccess ||
+        (e = to_device(P->d_tables.p, packed.data(), packed.size(), ctx->stream)) != cudaSuccess ||
         (e = P->scratch.ensure(std::max<size_t>(P->g[0].partials(), 1), std::max<size_t>(P->n_poses, 1), ctx->stream,
                                P->n_poses * (size_t)P->g[0].iface_words)) != cudaSuccess ||
-        (e = P->scratch.ensure_spill(std::max(group_spill_bytes(ctx, P->g[1], false),
-                                              group_spill_bytes(ctx, P->g[1], true)), ctx->stream)) != cudaSuccess ||
+        (e = P->scratch.ensure_spill(spill, ctx->stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) {
         delete P;
         return set_error(cuda_to_status(e), "plan setup: %s", cudaGetErrorString(e));
@@ -1341,9 +1350,9 @@ int lkg_plan_launch(lkg_plan* P, const double* d_poses, double* d_scores, double
         int st = sync_descriptors(P->ctx);
         if (st) return st;
     }
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < N_GROUPS; ++k) {
         if (P->g[k].ic.empty()) continue;
-        int st = launch_group(P->ctx, P->g[k], P->d_tables.as<char>() + (k ? P->b0 : 0), P->scratch, d_poses,
+        int st = launch_group(P->ctx, P->g[k], P->d_tables.as<char>() + P->off[k], P->scratch, d_poses,
                               d_scores, d_parts, 0, 0, nullptr, nullptr);
         if (st) return st;
     }
@@ -1355,9 +1364,9 @@ int lkg_plan_launch(lkg_plan* P, const double* d_poses, double* d_scores, double
 namespace lkg {
 int plan_launch_masked(lkg_plan* P, const double* d_poses, double* d_scores, const unsigned char* d_mask) {
     if (!P || !d_poses || !d_scores) return set_error(LKG_ERR_ARG, "bad plan launch");
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < N_GROUPS; ++k) {
         if (P->g[k].ic.empty()) continue;
-        int st = launch_group(P->ctx, P->g[k], P->d_tables.as<char>() + (k ? P->b0 : 0), P->scratch, d_poses,
+        int st = launch_group(P->ctx, P->g[k], P->d_tables.as<char>() + P->off[k], P->scratch, d_poses,
                               d_scores, nullptr, 0, 0, nullptr, nullptr, d_mask);
         if (st) return st;
     }
@@ -1387,7 +1396,8 @@ int lkg_plan_capture(lkg_plan* P, const double* d_poses, double* d_scores, doubl
     LKG_CK(cudaGraphInstantiate(&P->exec, g, 0), "graph instantiate");
     P->captured_cx = ctx->d_cx.p;
     P->captured_version = ctx->cx_version;
-    P->captured_launches = n_launches * ((P->g[0].ic.empty() ? 0 : 1) + (P->g[1].ic.empty() ? 0 : 1));
+    P->captured_launches = 0;
+    for (const Group& G : P->g) P->captured_launches += G.ic.empty() ? 0 : n_launches;
     return set_ok();
 }
 

@@ -88,7 +88,7 @@ struct ComplexRec {
     int n_cells = 0;
 };
 
-struct Occupancy { int threads = 0, hcap = 0, blocks = 0; };
+struct Occupancy { int threads = 0, hcap = 0, group = 0, blocks = 0; };
 
 // per-launch scratch: per-unit partial sums, per-pose counters, the work
 // counter and the status word (counters reset themselves after a launch)
@@ -113,12 +113,18 @@ inline cudaError_t to_device(void* dst, const void* src, size_t bytes, cudaStrea
     return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
 }
 
+// A batch's launch groups: the tile kernels', and the fused desolvation's for
+// ligands searched as the context's groups and for small ones of a context with
+// groups of 8 (scan()), which are searched by eights.
+constexpr int N_GROUPS = 3;
+
 // one launch group's item tables: (complex, first pose, pose count) per item
-// and cumulative work units; `kind` 0 = tile kernels, 1 = fused desolvation.
+// and cumulative work units; `kind` 0 = tile kernels, 1 = fused desolvation,
+// `group`: ligand atoms searched together.
 // sub > 0: the fast warp kernel takes units of `sub` ligand groups instead of
 // tiles (ws: cumulative units, g0: cumulative group partials per item)
 struct Group {
-    int kind = 0;
+    int kind = 0, group = 0;
     std::vector<int> ic, ip0, inp;
     std::vector<long long> w0{0};
     int sub = 0;
@@ -142,11 +148,16 @@ struct lkg_ctx {
     int precision = LKG_PREC_FAST;
     int tile = 128;                 // ligand atoms per work unit
     int group = 8;                  // ligand atoms per candidate-search group
-    // groups of 8 are searched two at a time: the cell rows, the set-up and the
-    // reductions cost the same for 16 atoms, and the candidate lists are per
-    // quad either way (1800 vdw poses 817 -> 729 us, 3000 poses with restraints
-    // 1715 -> 1489, 200 dna poses 150 -> 137)
-    int scan() const { return group == 8 ? 16 : group; }
+    // atoms of a ligand of n that are searched together.  Groups of 8 go two at
+    // a time: the cell rows, the set-up and the reductions cost the same for 16
+    // atoms, and the candidate lists are per quad either way (1800 vdw poses 817
+    // -> 729 us, 3000 poses with restraints 1715 -> 1489, 200 dna poses 150 ->
+    // 137).  Not those of a small cpydock ligand, whose groups are shared by the
+    // 8 warps of the pose's block: 3000 poses by eights / sixteens, ms, at chain
+    // and at protein density: 40 atoms 0.14 / 0.18 and 0.23 / 0.34, 300 atoms
+    // 0.48 / 0.51 and 0.94 / 1.02, 700 0.92 / 0.93 and 2.0 / 2.1, 800 1.05 / 1.02
+    // and 2.2 / 2.4, 1300 1.54 / 1.47 and 3.7 / 3.6
+    int scan(bool desolv, int n) const { return group != 8 ? group : (desolv && n <= 700 ? 8 : 16); }
     int desolv_threads = 512;
     float cell_h = 0.f;             // receptor cell edge in y and z (A); 0: per family
     int xsub = 0;                   // x sub-cells per cell edge; 0: per family
@@ -163,7 +174,7 @@ struct lkg_ctx {
     lkg::DBuf d_poses, d_scores, d_parts;
     lkg::HBuf h_poses, h_out, h_status;
     int64_t launches = 0;
-    lkg::Occupancy occ_tiles[2], occ_desolv[2];
+    lkg::Occupancy occ_tiles[2], occ_desolv[2][2];
     bool noalloc_used = false;      // lkg_score_device_noalloc ran on this context (its status word is checked)
     bool setup_on_device = true;    // receptor cell sort and packing on the GPU (false: the host build)
     bool stage_tma = false;         // plain warp kernel: candidates staged by bulk copies (measured alternative)
@@ -219,7 +230,7 @@ int check_status_word(int* d_status, cudaStream_t s);
 // status word of the no-allocation entry point's array on the context's device
 int noalloc_check_status(lkg_ctx* ctx);
 // item tables of the two launch groups for a batch
-int build_groups(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, Group g[2], size_t* n_poses);
+int build_groups(lkg_ctx* ctx, int n_items, const int* ids, const int* counts, Group g[N_GROUPS], size_t* n_poses);
 int sync_descriptors(lkg_ctx* ctx);
 // persistent grid of a launch group at the given precision
 long long group_blocks(lkg_ctx* ctx, const Group& g, bool exact);

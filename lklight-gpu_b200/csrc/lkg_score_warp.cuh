@@ -46,8 +46,9 @@ constexpr int WK_THREADS = 128;   // 4 independent warps per block
 // of a 1300-atom ligand on 12,600 atoms at protein density, ms at 128 / 160 /
 // 192 / 256 / 384: groups of 4 (one list): 2.94 / 2.89 / 2.84 / 2.80 / 2.76;
 // groups of 16 (four): 2.04 / 1.99 / 2.00 / 2.02 / 2.18; groups of 32 (eight):
-// 2.35 / 2.45 / 2.41 / 2.65 / 3.59.
-template <int G> constexpr int W_LIST = G == 4 ? 256 : 192;
+// 2.35 / 2.45 / 2.41 / 2.65 / 3.59.  Groups of 8 (cpydock, 300 atoms): 0.94 at
+// 192 and at 256.
+template <int G> constexpr int W_LIST = G <= 8 ? 256 : 192;
 
 // resident blocks per SM the register budget is sized for: 72 registers (a
 // few spills in the cold parts).  Sixteen complexes of 2,000 poses: 12.5 ms at
