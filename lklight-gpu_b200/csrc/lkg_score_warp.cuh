@@ -46,14 +46,17 @@ constexpr int WK_THREADS = 128;   // 4 independent warps per block
 // of a 1300-atom ligand on 12,600 atoms at protein density, ms at 128 / 160 /
 // 192 / 256 / 384: groups of 4 (one list): 2.94 / 2.89 / 2.84 / 2.80 / 2.76;
 // groups of 16 (four): 2.04 / 1.99 / 2.00 / 2.02 / 2.18; groups of 32 (eight):
-// 2.35 / 2.45 / 2.41 / 2.65 / 3.59.  Groups of 8 (cpydock, 300 atoms): 0.94 at
-// 192 and at 256.
-template <int G> constexpr int W_LIST = G <= 8 ? 256 : 192;
+// 2.35 / 2.45 / 2.41 / 2.65 / 3.59, 2.44 at 96.  Groups of 8 (cpydock, 300
+// atoms): 0.94 at 192 and at 256.
+template <int G> constexpr int W_LIST = G <= 8 ? 256 : (G == 32 ? 128 : 192);
 
 // resident blocks per SM the register budget is sized for: 72 registers (a
 // few spills in the cold parts).  Sixteen complexes of 2,000 poses: 12.5 ms at
-// 5 blocks, 12.4 at 6, 12.1 at 7, 12.5 at 8.
-constexpr int WK_BLOCKS = 7;
+// 5 blocks, 12.4 at 6, 12.1 at 7, 12.5 at 8.  Groups of 32, whose lists leave
+// room for no more: 5 (3000 vdw poses of 300 atoms on 5000 at chain density, ms
+// at 5 / 6 / 7 blocks: 0.255 / 0.266 / 0.289 with 7 A cells, 0.291 / 0.313 /
+// 0.360 with 2.5 A; 1300 atoms on 12,600 at protein density 2.17 / 2.20 / 2.34).
+template <int G> constexpr int WK_BLOCKS = G == 32 ? 5 : 7;
 // f64 mode: bound by the latency of its f64 chains, so more warps win over
 // fewer spills (200 poses: 440 us at 4 blocks, 399 at 5, 387 at 6, 370 at 7,
 // 360 at 8)
@@ -922,7 +925,7 @@ __device__ __forceinline__ void w_groups(const ComplexDev& c, WSlots<G>& W, WDes
 // NP: near pairs are counted (launches with parts)
 // EXACT: f64 pair math in the reference's operation order
 template <int G, bool IFACE, bool NP, bool STAGE = false, bool EXACT = false>
-__global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCKS) k_score_warp(const __grid_constant__ LaunchParams p) {
+__global__ void __launch_bounds__(WK_THREADS, EXACT ? WK_BLOCKS_EXACT : WK_BLOCKS<G>) k_score_warp(const __grid_constant__ LaunchParams p) {
     static_assert(G == 4 || G == 16 || G == 32, "group size");
     static_assert(!(STAGE && (IFACE || EXACT)), "the staged variant is the plain kernel's");
     constexpr unsigned FULL = 0xffffffffu;
